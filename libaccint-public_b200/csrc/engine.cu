@@ -27,6 +27,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -336,6 +337,81 @@ int ensure_scratch(lai_engine* E, size_t doubles) {
   return LAI_OK;
 }
 
+namespace {
+std::mutex g_lane_mutex;
+std::vector<LaneSet>& lane_pool() {  // never destroyed: the streams go with the CUDA context
+  static auto* pool = new std::vector<LaneSet>;
+  return *pool;
+}
+void destroy_lanes(LaneSet& set) {
+  for (auto e : set.ev)
+    if (e) cudaEventDestroy(e);
+  for (auto s : set.side)
+    if (s) cudaStreamDestroy(s);
+  set = LaneSet{};
+}
+}  // namespace
+
+int acquire_lanes(LaneSet& out) {
+  {
+    std::lock_guard<std::mutex> lock(g_lane_mutex);
+    if (!lane_pool().empty()) {
+      out = std::move(lane_pool().back());
+      lane_pool().pop_back();
+      return LAI_OK;
+    }
+  }
+  out.side.assign(kLanes - 1, nullptr);
+  out.ev.assign(kLanes, nullptr);
+  for (auto& s : out.side) LAI_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  for (auto& e : out.ev) LAI_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return LAI_OK;
+}
+
+// Work still queued on the set's streams was joined to the caller's stream, and the next
+// engine's work on them simply follows it.
+void release_lanes(LaneSet& set) {
+  if (set.side.size() != (size_t)kLanes - 1 || set.ev.size() != (size_t)kLanes || !set.ev.back())
+    return destroy_lanes(set);
+  std::lock_guard<std::mutex> lock(g_lane_mutex);
+  if (lane_pool().size() >= kPooledLaneSets) return destroy_lanes(set);
+  lane_pool().push_back(std::move(set));
+  set = LaneSet{};
+}
+
+LaunchLanes::LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread) : E_(E), main_(stream), load_(1, 0.0) {
+  E->fork_stream = stream;
+  if (!spread || E->lanes.side.empty()) return;
+  if (cudaEventRecord(E->lanes.ev[0], stream) != cudaSuccess) return;  // one lane: the caller's stream
+  load_.resize(E->lanes.side.size() + 1, -1.0);
+}
+
+cudaError_t LaunchLanes::pick(double work, cudaStream_t* s) {
+  size_t best = 0;
+  for (size_t i = 1; i < load_.size(); ++i)
+    if (std::max(load_[i], 0.0) < load_[best]) best = i;
+  *s = best ? E_->lanes.side[best - 1] : main_;
+  if (load_[best] < 0.0) {
+    load_[best] = 0.0;
+    if (cudaError_t e = cudaStreamWaitEvent(*s, E_->lanes.ev[0], 0)) return e;
+  }
+  load_[best] += work;
+  return cudaSuccess;
+}
+
+cudaError_t LaunchLanes::join() {
+  cudaError_t rc = cudaSuccess;
+  for (size_t i = 1; i < load_.size(); ++i) {
+    if (load_[i] < 0.0) continue;
+    cudaError_t e = cudaEventRecord(E_->lanes.ev[i], E_->lanes.side[i - 1]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(main_, E_->lanes.ev[i], 0);
+    if (e != cudaSuccess) rc = e;
+  }
+  load_.assign(1, 0.0);
+  E_->fork_stream = nullptr;
+  return rc;
+}
+
 // Launches the kernel of the block's class.  fp32 asks for the FP32 variant; the
 // classes without one (generic kernel) run in FP64, and *ran_fp32 says which ran.
 int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs& args,
@@ -382,8 +458,9 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
   }
   const size_t need = lai::generic_global_scratch_doubles(la, lb, lc, ld, E->num_sms);
   if (int rc = ensure_scratch(E, need)) return rc;
-  const int rc = lai::launch_generic(blk, args, E->tab, E->stream, E->d_scratch.as<double>(),
-                                     E->scratch_doubles, E->num_sms);
+  // one scratch buffer: launches that use it follow one another on the caller's stream
+  const int rc = lai::launch_generic(blk, args, E->tab, E->fork_stream ? E->fork_stream : E->stream,
+                                     E->d_scratch.as<double>(), E->scratch_doubles, E->num_sms);
   if (rc < 0) return fail(LAI_ECUDA, std::string("generic launch failed: ") +
                                          cudaGetErrorString(cudaGetLastError()));
   return LAI_OK;
@@ -756,7 +833,10 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
     LAI_CUDA_TRY(cudaMemsetAsync(E->d_prof_prims.p, 0, E->d_prof_prims.bytes, stream));
   }
   E->prof_n = 0;
-  for (size_t b = 0; b < E->blocks.size(); ++b) {
+  // profiled builds time every launch by itself, in block order on one stream
+  LaunchLanes lanes(E, stream, !o.profile);
+  for (size_t i = 0; i < E->blocks.size(); ++i) {
+    const size_t b = o.profile ? i : (size_t)E->launch_order[i];
     const auto& bp = *E->blocks[b];
     for (int part = 0; part < nparts; ++part) {
       // part 0: the whole block (FP64), or its FP64 prefix when mixed; part 1: the
@@ -777,6 +857,10 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
       args.prim_count = o.profile ? E->d_prof_prims.as<unsigned long long>() + E->prof_n : nullptr;
       if (o.profile) LAI_CUDA_TRY(cudaEventRecord(E->prof_ev[2 * E->prof_n], stream));
       bool ran32 = false;
+      if (cudaError_t ce = lanes.pick(bp.alg_flops * (double)(hi - lo), &E->stream)) {
+        E->stream = saved;
+        return fail(LAI_ECUDA, std::string("lai_jk: ") + cudaGetErrorString(ce));
+      }
       if (int rc = launch_block(E, q, args, part == 1, &ran32, bp.tune)) { E->stream = saved; return rc; }
       if (o.profile) {
         LAI_CUDA_TRY(cudaEventRecord(E->prof_ev[2 * E->prof_n + 1], stream));
@@ -790,6 +874,8 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
       flops += bp.alg_flops * (double)(hi - lo);
     }
   }
+  E->stream = saved;
+  LAI_CUDA_TRY(lanes.join());
   const int64_t nn = (int64_t)elems;
   if (nn > 0) {
     if (batched)
@@ -803,7 +889,6 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
   }
   LAI_CUDA_TRY(cudaGetLastError());
   if (timed) LAI_CUDA_TRY(cudaEventRecord(E->ev1, stream));
-  E->stream = saved;
   if (rep) {
     rep->quartets_fp64 = nq - nq32;
     rep->quartets_fp32 = nq32;
@@ -916,6 +1001,7 @@ int create_engine(const lai_basis* basis, std::unique_ptr<lai_basis> merged, con
   LAI_CUDA_TRY(cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking));
   LAI_CUDA_TRY(cudaEventCreate(&E->ev0));
   LAI_CUDA_TRY(cudaEventCreate(&E->ev1));
+  if (int rc = acquire_lanes(E->lanes)) return rc;
   {
     std::vector<double> coef(RYS_COEF_H, RYS_COEF_H + RYS_COEF_LEN);
     std::vector<double> hx(RYS_HERM_X2_H, RYS_HERM_X2_H + RYS_HERM_LEN);
@@ -942,6 +1028,12 @@ int create_engine(const lai_basis* basis, std::unique_ptr<lai_basis> merged, con
   if (int rc = compute_schwarz(E.get())) return rc;
   if (int rc = compute_prim_schwarz(E.get())) return rc;
   if (int rc = sort_and_screen(E.get())) return rc;
+  E->launch_order.resize(E->blocks.size());
+  std::iota(E->launch_order.begin(), E->launch_order.end(), 0);
+  std::stable_sort(E->launch_order.begin(), E->launch_order.end(), [&](int x, int y) {
+    return E->blocks[x]->alg_flops * (double)E->blocks[x]->total >
+           E->blocks[y]->alg_flops * (double)E->blocks[y]->total;
+  });
   *out = E.release();
   return LAI_OK;
 }

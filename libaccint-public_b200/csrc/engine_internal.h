@@ -75,6 +75,19 @@ struct lai_basis {
 namespace lai {
 namespace host {
 
+// The extra streams of an engine's builds (LaunchLanes): lane 0 is the caller's stream,
+// lane i side[i - 1].  Creating them takes about 0.4 ms, which would be a sixth of a
+// small engine's set-up, so a destroyed engine's set goes back to a process-wide pool
+// (at most kPooledLaneSets kept; mutex) and the next engine takes it.
+struct LaneSet {
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> ev;        // [0] fork, [i] end of side[i - 1]
+};
+constexpr int kLanes = 8;
+constexpr size_t kPooledLaneSets = 4;
+int acquire_lanes(LaneSet& out);
+void release_lanes(LaneSet& set);
+
 struct PairClassHost {
   int la, lb, Ka, Kb;
   double qprim_max = 0.0;
@@ -132,6 +145,7 @@ struct ClassPairBlock {
 }  // namespace lai
 
 struct lai_engine {
+  ~lai_engine();
   const lai_basis* basis = nullptr;
   // batched engines: the merged basis (owned) and the per-system layout of the
   // packed D/J/K arrays (block s = nbf_s x nbf_s at element offset sys_off[s])
@@ -191,16 +205,22 @@ struct lai_engine {
   std::vector<int64_t> prof_quartets;
   lai::host::DevBuf d_prof_prims;
   int prof_n = 0;
-  ~lai_engine() {
-    release_graph();
-    for (auto e : prof_ev) cudaEventDestroy(e);
-    classes.clear();
-    blocks.clear();
-    if (ev0) cudaEventDestroy(ev0);
-    if (ev1) cudaEventDestroy(ev1);
-    if (stream) cudaStreamDestroy(stream);
-  }
+  // streams the independent class-pair launches of one build are spread over
+  lai::host::LaneSet lanes;
+  cudaStream_t fork_stream = nullptr; // caller's stream while a build is spread over lanes
+  std::vector<int> launch_order;      // blocks by descending estimated work
 };
+
+inline lai_engine::~lai_engine() {
+  release_graph();
+  for (auto e : prof_ev) cudaEventDestroy(e);
+  classes.clear();
+  blocks.clear();
+  if (ev0) cudaEventDestroy(ev0);
+  if (ev1) cudaEventDestroy(ev1);
+  lai::host::release_lanes(lanes);
+  if (stream) cudaStreamDestroy(stream);
+}
 
 namespace lai {
 namespace host {
@@ -212,6 +232,29 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
                  bool fp32 = false, bool* ran_fp32 = nullptr, lai::LaunchTune tune = lai::LaunchTune{});
 lai::QuartetBlock make_block(const lai_engine* E, const ClassPairBlock& b);
 int ensure_scratch(lai_engine* E, size_t doubles);
+
+// Spreads independent launches over the engine's lanes: pick(w) returns the stream of
+// the lane with the least estimated work so far; join() makes the caller's stream wait
+// for all of them.  The class-pair launches of one build only add to J'/K' (or the
+// gradient) with atomics, so their order does not matter, and most of them do not fill
+// the device alone: H2O / cc-pVQZ takes 666 launches, most with a few warps.  The blocks
+// go out by descending estimated work, so that the small launches fill the large ones'
+// last waves.  kLanes is the number of hardware queues a process gets by default; more
+// streams would share them.  One stream -> eight (device time of a build): H2O/STO-3G
+// 106 -> 49 us, H2O/cc-pVQZ 320 -> 120 ms, (H2O)16/cc-pVDZ 53.2 -> 39.3 ms,
+// (H2O)64/cc-pVDZ 1505 -> 1390 ms; (H2O)6/cc-pVDZ gradient 82.5 -> 30.5 ms.
+class LaunchLanes {
+ public:
+  LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread);
+  ~LaunchLanes() { join(); }
+  cudaError_t pick(double work, cudaStream_t* s);
+  cudaError_t join();
+
+ private:
+  lai_engine* E_;
+  cudaStream_t main_;
+  std::vector<double> load_;   // estimated work per lane; < 0: not forked yet
+};
 double alg_work(int la, int lb, int lc, int ld, int Ka, int Kb, int Kc, int Kd);
 
 }  // namespace host

@@ -46,11 +46,15 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
   if (!engine || !d_D || !d_grad) return fail(LAI_EINVAL, "lai_jk_gradient_device: null argument");
   LAI_CUDA_TRY(cudaSetDevice(engine->device));
   if (int rc = ensure_atoms(engine)) return rc;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  LAI_CUDA_TRY(cudaMemsetAsync(d_grad, 0, sizeof(double) * 3 * engine->natom, s));
+  cudaStream_t stream_of_call = static_cast<cudaStream_t>(stream);
+  LAI_CUDA_TRY(cudaMemsetAsync(d_grad, 0, sizeof(double) * 3 * engine->natom, stream_of_call));
   const int nbf = (int)engine->basis->nbf;
-  for (const auto& bp : engine->blocks) {
+  LaunchLanes lanes(engine, stream_of_call, true);
+  for (const int b : engine->launch_order) {
+    const auto& bp = engine->blocks[b];
     const lai::QuartetBlock q = make_block(engine, *bp);
+    cudaStream_t s = stream_of_call;
+    LAI_CUDA_TRY(lanes.pick(bp->alg_flops * (double)bp->total, &s));
     const int rs = lai::launch_grad_small(q, d_D, nbf, engine->d_shell_atom.as<int>(), d_grad, engine->prim_eps,
                                           engine->tab, s, engine->num_sms);
     if (rs == 0) continue;
@@ -59,12 +63,14 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
     const size_t need = lai::grad_global_scratch_doubles(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb,
                                                          engine->num_sms);
     if (int rc = ensure_scratch(engine, need)) return rc;
+    if (need) s = stream_of_call;  // one scratch buffer: its users follow one another
     const int rc = lai::launch_grad(q, d_D, nbf, engine->d_shell_atom.as<int>(), d_grad, engine->prim_eps,
                                     engine->tab, s, engine->d_scratch.as<double>(), engine->scratch_doubles,
                                     engine->num_sms);
     if (rc < 0)
       return fail(LAI_ECUDA, std::string("gradient launch failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
+  LAI_CUDA_TRY(lanes.join());
   return LAI_OK;
 }
 
