@@ -362,7 +362,7 @@ LAI_API int64_t lai_engine_quartet_count(lai_engine* engine);
 /* Autotuner: times every thread-per-quartet class launch of the engine under a
  * few launch configurations (lanes per quartet 1..8, chunks per super-chunk 1, 4,
  * 16), and every other class launch under each kernel family that covers it
- * (warp-per-quartet, bra-sliced, tiled), on the device density d_D, and keeps the
+ * (block-per-quartet, bra-sliced, tiled), on the device density d_D, and keeps the
  * fastest for later builds.
  * ms_before/ms_after (may be NULL): summed launch times with the built-in
  * heuristic and with the chosen configurations.  Synchronizes `stream`. */
@@ -370,7 +370,7 @@ LAI_API int lai_engine_autotune(lai_engine* engine, const double* d_D, void* str
                                 double* ms_after);
 /* The launch table: per class-pair block, 10 ints: la, lb, lc, ld, bra and ket
  * primitive pairs per shell pair, quartets (capped at INT32_MAX), tuned lanes per
- * quartet (or -1 warp-per-quartet, -2 tiled, -3 bra-sliced kernel for the classes
+ * quartet (or -2 tiled, -3 bra-sliced, -4 block-per-quartet kernel for the classes
  * outside the thread-per-quartet set) and chunks per super-chunk (0 = heuristic),
  * quartets / 1000.  Returns
  * the block count; rows may be NULL to query it. */

@@ -425,23 +425,23 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
                                            cudaGetErrorString(cudaGetLastError()));
     return LAI_OK;
   }
-  // the other classes: warp-per-quartet, bra-sliced or tiled kernel, as tuned for
-  // this block (lai_engine_autotune) or by the measured per-class default; FP32
-  // requests go to the sliced kernel where it exists, else to the warp-per-quartet
-  // kernel's FP32 variant (d and f classes; the tiled and generic kernels are FP64
-  // only)
-  int kern = tune.kernel != lai::KERNEL_DEFAULT ? tune.kernel : lai::default_kernel(la, lb, lc, ld);
-  if (fp32 && lai::sliced_class_supported(la, lb, lc, ld)) kern = lai::KERNEL_SLICED;
-  else if (fp32 && lai::warpq_class_supported(la, lb, lc, ld)) kern = lai::KERNEL_WARPQ;
-  if (kern == lai::KERNEL_WARPQ) {
-    const int rc = lai::launch_warpq(blk, args, E->tab, E->stream, E->num_sms, fp32);
-    if (rc == 1) {
-      if (ran_fp32) *ran_fp32 = true;
+  // the other classes: block-per-quartet, bra-sliced or tiled kernel, as tuned for this
+  // block (lai_engine_autotune) or by default_kernel; FP32 requests go to the sliced
+  // kernel where it exists, else to the block-per-quartet kernel's FP32 variant (the
+  // tiled and generic kernels are FP64 only).  The raw-integral and Schwarz modes run on
+  // the sliced and tiled kernels.
+  int kern = tune.kernel != lai::KERNEL_DEFAULT ? tune.kernel
+             : lai::default_kernel(la, lb, lc, ld, blk.total - blk.t_begin, E->num_sms);
+  if (fp32) kern = lai::sliced_class_supported(la, lb, lc, ld) ? lai::KERNEL_SLICED : lai::KERNEL_BLOCK;
+  if (kern == lai::KERNEL_BLOCK) {
+    const bool f32 = fp32 && lai::block_fp32_class(la, lb, lc, ld);
+    const int rc = lai::launch_blockq(blk, args, E->tab, E->stream, E->num_sms, f32);
+    if (rc == 0) {
+      if (ran_fp32) *ran_fp32 = f32;
       return LAI_OK;
     }
-    if (rc == 0) return LAI_OK;
-    if (rc < -1) return fail(LAI_ECUDA, std::string("warp-per-quartet launch failed: ") +
-                                            cudaGetErrorString(lai::warpq_launch_error()));
+    if (rc < -1) return fail(LAI_ECUDA, std::string("block-per-quartet launch failed: ") +
+                                            cudaGetErrorString(cudaGetLastError()));
   }
   if (kern != lai::KERNEL_TILED && lai::sliced_class_supported(la, lb, lc, ld)) {
     const int rc = lai::launch_sliced(blk, args, E->tab, E->stream, fp32, E->num_sms);
@@ -1394,12 +1394,10 @@ int lai_engine_autotune(lai_engine* engine, const double* d_D, void* stream, dou
     if ((rc = time_launch(q, bp->tune, &base))) break;
     before += base;
     if (!lai::small_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb)) {
-      // kernel family: warp-per-quartet, bra-sliced, tiled
+      // kernel family: block-per-quartet, bra-sliced, tiled
       lai::LaunchTune best = bp->tune;
       float best_ms = base;
-      for (int k : {lai::KERNEL_WARPQ, lai::KERNEL_SLICED, lai::KERNEL_TILED}) {
-        if (k == lai::KERNEL_WARPQ && !lai::warpq_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb))
-          continue;
+      for (int k : {lai::KERNEL_BLOCK, lai::KERNEL_SLICED, lai::KERNEL_TILED}) {
         if (k == lai::KERNEL_SLICED && !lai::sliced_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb))
           continue;
         lai::LaunchTune t;

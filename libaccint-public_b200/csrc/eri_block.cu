@@ -1,0 +1,58 @@
+// Dispatch of the block-per-quartet kernel (eri_block_impl.cuh) over its kets, which are
+// instantiated in eri_block_k*.cu, and the choice of kernel family for the classes
+// outside the thread-per-quartet set.
+#include <cuda_runtime.h>
+
+#include "eri_kernels.h"
+
+namespace lai {
+namespace block_detail {
+template <int LC, int LD, int F0, int F1, typename R>
+int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
+                 int num_sms);
+}  // namespace block_detail
+
+int launch_blockq(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
+                  int num_sms, bool fp32) {
+  if (args.mode != MODE_JK) return -1;
+  if (blk.total - blk.t_begin <= 0) return 0;
+  const int lc = blk.ket.la, ld = blk.ket.lb;
+#define K(c, d, f0, f1)                                                                               \
+  if (lc == c && ld == d) {                                                                           \
+    if constexpr (c < 4)                                                                              \
+      if (fp32) return block_detail::launch_range<c, d, f0, f1, float>(blk, args, tab, stream, num_sms); \
+    if (const int rc = block_detail::launch_range<c, d, f0, f1, double>(blk, args, tab, stream, num_sms)) return rc; \
+  }
+  K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 2, 4) K(3, 0, 3, 3)
+  K(3, 1, 3, 4) K(3, 2, 3, 5) K(3, 3, 3, 6) K(4, 0, 4, 4) K(4, 1, 4, 5) K(4, 2, 4, 6)
+  // more components than a thread's registers hold: two launches, each digests its part
+  K(4, 3, 4, 5) K(4, 3, 6, 7) K(4, 4, 4, 6) K(4, 4, 7, 8)
+#undef K
+  return 0;
+}
+
+// FP32 covers the d and f classes with at most 1152 contracted (e0|f0) integrals; the
+// larger ones, and the g classes, run in FP64 in a mixed-precision build.
+bool block_fp32_class(int la, int lb, int lc, int ld) {
+  return la <= 3 && ncart_range(la, la + lb) * ncart_range(lc, lc + ld) <= 1152;
+}
+
+// The block-per-quartet kernel, except large launches of the bra-sliced classes.  Those,
+// (dp|pp), (dp|dp) and (dd|ds), leave half of a block's threads without a row (16 of 32; 31
+// for (dd|) and their digestion is short: one launch of (dp|pp), C2H6/cc-pVQZ, 1.3e5
+// quartets of one primitive quartet, takes 0.248 ms on either kernel.  With fewer
+// quartets than the device holds blocks the block kernel, which splits a quartet, takes
+// them too: the same class in H2O/cc-pVQZ with 25 - 36 primitive quartets.
+//
+// What the block kernel replaced in the other classes was the tiled kernel (one warp per
+// quartet, its table and digestion sweeps repeated for every 512 integrals) and a
+// warp-per-quartet kernel with scattered (e0|f0) ownership.  Device time per class,
+// C6H14/cc-pVTZ, before -> now: (fd|dp) 21.6 -> 1.9 ms, (fp|dp) 23.1 -> 2.6, (fd|dd) 10.3
+// -> 0.8, (ff|fd) 8.1 -> 0.3, (dd|dp) 6.2 -> 3.1, (fp|ps) 4.4 -> 3.7; one (gg|gg) quartet
+// 74 ms -> 0.1 ms.  Whole builds: C6H14/cc-pVTZ 199 -> 90 ms, H2O/cc-pVQZ 120 -> 5.1 ms.
+int default_kernel(int la, int lb, int lc, int ld, int64_t nq, int num_sms) {
+  if (nq >= (int64_t)32 * num_sms && sliced_class_supported(la, lb, lc, ld)) return KERNEL_SLICED;
+  return KERNEL_BLOCK;
+}
+
+}  // namespace lai

@@ -17,9 +17,9 @@ struct LaunchTune {
   int ps = 0;
   int ksuper = 0;
   int kernel = 0;  // classes outside the thread-per-quartet set: 0 = default choice,
-                   // KERNEL_WARPQ, KERNEL_TILED or KERNEL_SLICED
+                   // KERNEL_TILED, KERNEL_SLICED or KERNEL_BLOCK
 };
-enum { KERNEL_DEFAULT = 0, KERNEL_WARPQ = 1, KERNEL_TILED = 2, KERNEL_SLICED = 3 };
+enum { KERNEL_DEFAULT = 0, KERNEL_TILED = 2, KERNEL_SLICED = 3, KERNEL_BLOCK = 4 };
 int launch_small(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,
                  cudaStream_t stream, bool fp32, int num_sms, LaunchTune tune = LaunchTune{});
 bool small_class_supported(int la, int lb, int lc, int ld);
@@ -29,21 +29,21 @@ int launch_sliced(const QuartetBlock& blk, const JKArgs& args, const RysTablesVi
                   cudaStream_t stream, bool fp32, int num_sms);
 bool sliced_class_supported(int la, int lb, int lc, int ld);
 
+// Kernel family of a J/K launch of nq quartets of a class outside the thread-per-quartet
+// set when no tuned choice exists (measured per class on B200: eri_block.cu).
+int default_kernel(int la, int lb, int lc, int ld, int64_t nq, int num_sms);
 // Warp-per-quartet kernel with lanes over the output integrals (eri_tiled.cu),
-// any class with l <= 4; 0 on success, -1 if the class does not fit shared memory.
-// Warp-per-quartet kernel compile-time specialised per class (J/K mode only).
-// Returns 0 when launched in FP64, 1 when fp32 asked for and got the FP32 variant
-// (d and f classes), -1 when the class is not instantiated (or the mode is not
-// J/K), < -1 on a CUDA error.
-int launch_warpq(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
-                 int num_sms, bool fp32 = false);
-cudaError_t warpq_launch_error();  // CUDA error of the last failed launch_warpq
-bool warpq_class_supported(int la, int lb, int lc, int ld);
-// Kernel family of a class outside the thread-per-quartet set when no tuned choice
-// exists (measured per class on B200: eri_warpq.cu).
-int default_kernel(int la, int lb, int lc, int ld);
+// any class with l <= 4, all modes; 0 on success, -1 if the class does not fit shared
+// memory.
 int launch_tiled(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
                  int num_sms);
+
+// Block-per-quartet kernel (eri_block.cu), any class with l <= 4, J/K mode only: 0 on
+// success, -1 for another mode, -3 on a CUDA error.
+// fp32 asks for the FP32 variant (block_fp32_class).
+int launch_blockq(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
+                  int num_sms, bool fp32);
+bool block_fp32_class(int la, int lb, int lc, int ld);
 
 // Warp-per-quartet generic kernel (eri_generic.cu), any class with l <= 4.
 int launch_generic(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,
