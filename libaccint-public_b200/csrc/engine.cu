@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <numeric>
@@ -35,18 +36,12 @@
 #include "../../include/libaccint_b200.h"
 #include "engine_internal.h"
 #include "eri_kernels.h"
-#include "rys_tables.inc"
-#include "fp32_tables.h"
 
 namespace lai {
 void spherical_forget_basis(const lai_basis* basis);  // spherical.cu
 }  // namespace lai
 
 using namespace lai::host;
-
-static_assert(RYS_DEG == lai::kRysDeg, "table degree mismatch");
-static_assert(BOYS_NM == lai::kBoysNM, "Boys table width mismatch");
-static_assert(BOYS_NGRID == lai::kBoysNGrid, "Boys grid mismatch");
 
 namespace lai {
 namespace host {
@@ -208,10 +203,11 @@ int build_classes(lai_engine* E) {
   const int ns = (int)sh.size();
   // class key -> index
   std::vector<std::array<int, 4>> keys;
+  std::map<std::array<int, 4>, int> index;
   auto class_of = [&](int la, int lb, int Ka, int Kb) {
     std::array<int, 4> k{la, lb, Ka, Kb};
-    for (size_t i = 0; i < keys.size(); ++i)
-      if (keys[i] == k) return (int)i;
+    const auto it = index.emplace(k, (int)keys.size());
+    if (!it.second) return it.first->second;
     keys.push_back(k);
     E->classes.push_back(std::make_unique<PairClassHost>());
     auto& c = *E->classes.back();
@@ -348,6 +344,9 @@ void destroy_lanes(LaneSet& set) {
     if (e) cudaEventDestroy(e);
   for (auto s : set.side)
     if (s) cudaStreamDestroy(s);
+  for (auto e : {set.t0, set.t1})
+    if (e) cudaEventDestroy(e);
+  if (set.main) cudaStreamDestroy(set.main);
   set = LaneSet{};
 }
 }  // namespace
@@ -365,13 +364,16 @@ int acquire_lanes(LaneSet& out) {
   out.ev.assign(kLanes, nullptr);
   for (auto& s : out.side) LAI_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   for (auto& e : out.ev) LAI_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  LAI_CUDA_TRY(cudaStreamCreateWithFlags(&out.main, cudaStreamNonBlocking));
+  LAI_CUDA_TRY(cudaEventCreate(&out.t0));
+  LAI_CUDA_TRY(cudaEventCreate(&out.t1));
   return LAI_OK;
 }
 
 // Work still queued on the set's streams was joined to the caller's stream, and the next
 // engine's work on them simply follows it.
 void release_lanes(LaneSet& set) {
-  if (set.side.size() != (size_t)kLanes - 1 || set.ev.size() != (size_t)kLanes || !set.ev.back())
+  if (set.side.size() != (size_t)kLanes - 1 || set.ev.size() != (size_t)kLanes || !set.t1)
     return destroy_lanes(set);
   std::lock_guard<std::mutex> lock(g_lane_mutex);
   if (lane_pool().size() >= kPooledLaneSets) return destroy_lanes(set);
@@ -466,214 +468,12 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
   return LAI_OK;
 }
 
-int compute_schwarz(lai_engine* E) {
-  // Diagonal quartets (ab|ab) of every pair: offsets[p] = p, qbegin[p] = p.
-  for (auto& cp : E->classes) {
-    auto& c = *cp;
-    const int n = c.n();
-    std::vector<int64_t> off(n + 1);
-    std::vector<int> qb(n);
-    for (int p = 0; p <= n; ++p) off[p] = p;
-    for (int p = 0; p < n; ++p) qb[p] = p;
-    DevBuf d_off, d_qb, d_out;
-    LAI_CUDA_TRY(upload(d_off, off));
-    LAI_CUDA_TRY(upload(d_qb, qb));
-    LAI_CUDA_TRY(d_out.alloc(sizeof(double) * n));
-    lai::QuartetBlock blk{};
-    blk.bra = blk.ket = c.view();
-    blk.offsets = d_off.as<int64_t>();
-    blk.qbegin = d_qb.as<int>();
-    blk.total = n;
-    blk.same_class = 1;
-    lai::JKArgs args{};
-    args.mode = lai::MODE_SCHWARZ;
-    args.schwarz_out = d_out.as<double>();
-    if (int rc = launch_block(E, blk, args)) return rc;
-    c.Q.resize(n);
-    LAI_CUDA_TRY(cudaMemcpyAsync(c.Q.data(), d_out.p, sizeof(double) * n, cudaMemcpyDeviceToHost,
-                                 E->stream));
-    LAI_CUDA_TRY(cudaStreamSynchronize(E->stream));
-  }
-  return LAI_OK;
-}
-
-// Primitive Schwarz bounds: every primitive pair of every shell pair is run as a
-// one-primitive pair through the diagonal kernel, q = sqrt(max |(a_p b_q|a_p b_q)|)
-// (contraction coefficients included).  By the Schwarz inequality a primitive
-// quartet contributes at most q_ab q_cd to any integral of its quartet.
-int compute_prim_schwarz(lai_engine* E) {
-  for (auto& cp : E->classes) {
-    auto& c = *cp;
-    const int n = c.n();
-    const int Kab = c.Ka * c.Kb;
-    const int ne = n * Kab;
-    if (ne == 0) continue;
-    PairClassHost pc;
-    pc.la = c.la; pc.lb = c.lb; pc.Ka = 1; pc.Kb = 1;
-    pc.sa.resize(ne); pc.sb.resize(ne); pc.fa.resize(ne); pc.fb.resize(ne);
-    pc.AB.resize(3 * (size_t)ne);
-    pc.Acen.resize(3 * (size_t)ne);
-    pc.prim.assign((size_t)lai::PF_COUNT * ne, 0.0);
-    for (int p = 0; p < n; ++p)
-      for (int t = 0; t < Kab; ++t) {
-        const int e = p * Kab + t;
-        pc.sa[e] = c.sa[p]; pc.sb[e] = c.sb[p]; pc.fa[e] = c.fa[p]; pc.fb[e] = c.fb[p];
-        for (int x = 0; x < 3; ++x) {
-          pc.AB[(size_t)x * ne + e] = c.AB[(size_t)x * n + p];
-          pc.Acen[(size_t)x * ne + e] = c.Acen[(size_t)x * n + p];
-        }
-        for (int f = 0; f < lai::PF_COUNT; ++f)
-          pc.prim[(size_t)f * ne + e] = c.prim[((size_t)f * Kab + t) * n + p];
-      }
-    if (int rc = upload_class(pc)) return rc;
-    std::vector<int64_t> off(ne + 1);
-    std::vector<int> qb(ne);
-    for (int e = 0; e <= ne; ++e) off[e] = e;
-    for (int e = 0; e < ne; ++e) qb[e] = e;
-    DevBuf d_off, d_qb, d_out;
-    LAI_CUDA_TRY(upload(d_off, off));
-    LAI_CUDA_TRY(upload(d_qb, qb));
-    LAI_CUDA_TRY(d_out.alloc(sizeof(double) * ne));
-    lai::QuartetBlock blk{};
-    blk.bra = blk.ket = pc.view();
-    blk.offsets = d_off.as<int64_t>();
-    blk.qbegin = d_qb.as<int>();
-    blk.total = ne;
-    blk.same_class = 1;
-    lai::JKArgs args{};
-    args.mode = lai::MODE_SCHWARZ;
-    args.schwarz_out = d_out.as<double>();
-    if (int rc = launch_block(E, blk, args)) return rc;
-    std::vector<double> q(ne);
-    LAI_CUDA_TRY(cudaMemcpyAsync(q.data(), d_out.p, sizeof(double) * ne, cudaMemcpyDeviceToHost,
-                                 E->stream));
-    LAI_CUDA_TRY(cudaStreamSynchronize(E->stream));
-    for (int p = 0; p < n; ++p)
-      for (int t = 0; t < Kab; ++t)
-        c.prim[((size_t)lai::PF_Q * Kab + t) * n + p] = q[(size_t)p * Kab + t];
-  }
-  return LAI_OK;
-}
-
-int sort_and_screen(lai_engine* E) {
-  const int ns = (int)E->basis->shells.size();
-  const bool batched = E->nsys > 1;
-  if (!batched) E->Q_all.assign((size_t)ns * ns, 0.0);  // (a full matrix only for one system)
-  double qmax = 0.0;
-  for (auto& cp : E->classes)
-    for (int p = 0; p < cp->n(); ++p) {
-      qmax = std::max(qmax, cp->Q[p]);
-      if (!batched) {
-        E->Q_all[(size_t)cp->sa[p] * ns + cp->sb[p]] = cp->Q[p];
-        E->Q_all[(size_t)cp->sb[p] * ns + cp->sa[p]] = cp->Q[p];
-      }
-    }
-  for (auto& cp : E->classes) {
-    auto& c = *cp;
-    const int n = c.n();
-    // pairs ordered by system, then by Schwarz bound (descending); pairs that pass
-    // with no partner dropped -- each system's kept pairs are a prefix of its segment
-    std::vector<int> idx;
-    idx.reserve(n);
-    for (int i = 0; i < n; ++i)
-      if (c.Q[i] * qmax >= E->thr) idx.push_back(i);
-    std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) {
-      return c.sys[x] != c.sys[y] ? c.sys[x] < c.sys[y] : c.Q[x] > c.Q[y];
-    });
-    const int keep = (int)idx.size();
-    const int Kab = c.Ka * c.Kb;
-    auto perm = [&](const std::vector<int>& v) {
-      std::vector<int> o(keep);
-      for (int i = 0; i < keep; ++i) o[i] = v[idx[i]];
-      return o;
-    };
-    std::vector<double> Q(keep), AB(3 * (size_t)keep), Acen(3 * (size_t)keep),
-        prim((size_t)lai::PF_COUNT * Kab * keep);
-    for (int i = 0; i < keep; ++i) {
-      Q[i] = c.Q[idx[i]];
-      for (int x = 0; x < 3; ++x) {
-        AB[(size_t)x * keep + i] = c.AB[(size_t)x * n + idx[i]];
-        Acen[(size_t)x * keep + i] = c.Acen[(size_t)x * n + idx[i]];
-      }
-      for (int f = 0; f < lai::PF_COUNT * Kab; ++f)
-        prim[(size_t)f * keep + i] = c.prim[(size_t)f * n + idx[i]];
-    }
-    // primitive pairs of each shell pair in descending primitive-Schwarz order
-    c.qprim_max = 0.0;
-    std::vector<int> tix(Kab);
-    std::vector<double> tmp(Kab);
-    for (int i = 0; i < keep; ++i) {
-      auto qat = [&](int t) { return prim[((size_t)lai::PF_Q * Kab + t) * keep + i]; };
-      std::iota(tix.begin(), tix.end(), 0);
-      std::stable_sort(tix.begin(), tix.end(), [&](int x, int y) { return qat(x) > qat(y); });
-      for (int f = 0; f < lai::PF_COUNT; ++f) {
-        for (int t = 0; t < Kab; ++t) tmp[t] = prim[((size_t)f * Kab + tix[t]) * keep + i];
-        for (int t = 0; t < Kab; ++t) prim[((size_t)f * Kab + t) * keep + i] = tmp[t];
-      }
-      c.qprim_max = std::max(c.qprim_max, qat(0));
-    }
-    c.sa = perm(c.sa); c.sb = perm(c.sb); c.fa = perm(c.fa); c.fb = perm(c.fb);
-    c.sys = perm(c.sys);
-    c.Q = std::move(Q); c.AB = std::move(AB); c.Acen = std::move(Acen); c.prim = std::move(prim);
-    c.seg.assign(E->nsys + 1, 0);
-    for (int i = 0, s = 0; s <= E->nsys; ++s) {
-      while (i < keep && c.sys[i] < s) ++i;
-      c.seg[s] = i;
-    }
-    c.batched = batched;
-    if (int rc = upload_class(c)) return rc;
-    if (batched) LAI_CUDA_TRY(upload(c.d_sys, c.sys));
-    {  // FP32 copy of the primitive-pair table for the FP32 kernels
-      std::vector<float> pf(c.prim.size());
-      for (size_t i = 0; i < pf.size(); ++i) pf[i] = (float)c.prim[i];
-      LAI_CUDA_TRY(upload(c.d_primf, pf));
-    }
-  }
-  // quartet blocks
-  const int nc = (int)E->classes.size();
-  for (int A = 0; A < nc; ++A)
-    for (int B = 0; B <= A; ++B) {
-      const auto& ca = *E->classes[A];
-      const auto& cb = *E->classes[B];
-      if (ca.n() == 0 || cb.n() == 0) continue;
-      auto blk = std::make_unique<ClassPairBlock>();
-      blk->bra = A;
-      blk->ket = B;
-      blk->offsets.resize(ca.n() + 1);
-      blk->offsets[0] = 0;
-      if (batched) blk->qbegin.resize(ca.n());
-      for (int p = 0; p < ca.n(); ++p) {
-        // largest prefix of the bra pair's system segment of the ket list with
-        // Q_p * Q_q >= thr (the whole list for a single system)
-        const int s0 = cb.seg[ca.sys[p]], s1 = cb.seg[ca.sys[p] + 1];
-        int lo = s0, hi = s1;
-        while (lo < hi) {
-          const int mid = (lo + hi) / 2;
-          if (ca.Q[p] * cb.Q[mid] >= E->thr) lo = mid + 1; else hi = mid;
-        }
-        int cnt = lo - s0;
-        if (A == B) cnt = std::min(cnt, p - s0 + 1);  // canonical q <= p (same segment)
-        blk->offsets[p + 1] = blk->offsets[p] + cnt;
-        if (batched) blk->qbegin[p] = s0;
-      }
-      blk->total = blk->offsets[ca.n()];
-      if (blk->total == 0) continue;
-      if (batched) LAI_CUDA_TRY(upload(blk->d_qbegin, blk->qbegin));
-      blk->alg_flops = alg_work(ca.la, ca.lb, cb.la, cb.lb, ca.Ka, ca.Kb, cb.Ka, cb.Kb);
-      blk->flops_per_prim = alg_per_prim(ca.la, ca.lb, cb.la, cb.lb);
-      blk->flops_per_quartet = alg_per_quartet(ca.la, ca.lb, cb.la, cb.lb);
-      LAI_CUDA_TRY(upload(blk->d_offsets, blk->offsets));
-      E->blocks.push_back(std::move(blk));
-    }
-  return LAI_OK;
-}
-
 lai::QuartetBlock make_block(const lai_engine* E, const ClassPairBlock& b) {
   lai::QuartetBlock q{};
   q.bra = E->classes[b.bra]->view();
   q.ket = E->classes[b.ket]->view();
-  q.offsets = b.d_offsets.as<int64_t>();
-  q.qbegin = b.qbegin.empty() ? nullptr : b.d_qbegin.as<int>();
+  q.offsets = b.dev_offsets;
+  q.qbegin = b.dev_qbegin;
   q.total = b.total;
   q.same_class = (b.bra == b.ket);
   return q;
@@ -998,36 +798,13 @@ int create_engine(const lai_basis* basis, std::unique_ptr<lai_basis> merged, con
   E->thr = o.schwarz_threshold;
   E->prim_eps = o.prim_threshold < 0.0 ? 1e-3 * o.schwarz_threshold : o.prim_threshold;
   LAI_CUDA_TRY(cudaDeviceGetAttribute(&E->num_sms, cudaDevAttrMultiProcessorCount, o.device));
-  LAI_CUDA_TRY(cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking));
-  LAI_CUDA_TRY(cudaEventCreate(&E->ev0));
-  LAI_CUDA_TRY(cudaEventCreate(&E->ev1));
   if (int rc = acquire_lanes(E->lanes)) return rc;
-  {
-    std::vector<double> coef(RYS_COEF_H, RYS_COEF_H + RYS_COEF_LEN);
-    std::vector<double> hx(RYS_HERM_X2_H, RYS_HERM_X2_H + RYS_HERM_LEN);
-    std::vector<double> hw(RYS_HERM_W_H, RYS_HERM_W_H + RYS_HERM_LEN);
-    std::vector<double> bg(BOYS_GRID_H, BOYS_GRID_H + BOYS_NGRID * BOYS_NM);
-    LAI_CUDA_TRY(upload(E->d_coef, coef));
-    LAI_CUDA_TRY(upload(E->d_hx2, hx));
-    LAI_CUDA_TRY(upload(E->d_hw, hw));
-    LAI_CUDA_TRY(upload(E->d_boys, bg));
-    // FP32 tables of the packed FP32 kernels, derived from the FP64 ones
-    std::vector<float> bf((size_t)lai::kBoysF32Rows * lai::kBoysF32Stride), rf(2 * (size_t)lai::kRysF32Len);
-    lai::build_boys_f32(BOYS_GRID_H, bf.data());
-    lai::build_rys_f32(RYS_COEF_H, rf.data());
-    LAI_CUDA_TRY(upload(E->d_boys_f32, bf));
-    LAI_CUDA_TRY(upload(E->d_rys_f32, rf));
-    E->tab = {E->d_coef.as<double>(), E->d_hx2.as<double>(), E->d_hw.as<double>(),
-              E->d_boys.as<double>(), E->d_boys_f32.as<float>(), E->d_rys_f32.as<float>()};
-  }
+  E->stream = E->lanes.main;
+  E->ev0 = E->lanes.t0;
+  E->ev1 = E->lanes.t1;
+  if (int rc = setup_tables(E.get())) return rc;
   if (int rc = build_classes(E.get())) return rc;
-  for (auto& c : E->classes) {
-    fill_pair_data(basis, *c);
-    if (int rc = upload_class(*c)) return rc;
-  }
-  if (int rc = compute_schwarz(E.get())) return rc;
-  if (int rc = compute_prim_schwarz(E.get())) return rc;
-  if (int rc = sort_and_screen(E.get())) return rc;
+  if (int rc = setup_pairs(E.get())) return rc;
   E->launch_order.resize(E->blocks.size());
   std::iota(E->launch_order.begin(), E->launch_order.end(), 0);
   std::stable_sort(E->launch_order.begin(), E->launch_order.end(), [&](int x, int y) {

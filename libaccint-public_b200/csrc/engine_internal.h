@@ -75,13 +75,15 @@ struct lai_basis {
 namespace lai {
 namespace host {
 
-// The extra streams of an engine's builds (LaunchLanes): lane 0 is the caller's stream,
-// lane i side[i - 1].  Creating them takes about 0.4 ms, which would be a sixth of a
+// An engine's streams and events.  Builds (LaunchLanes) run on the caller's stream, lane 0,
+// and side[i - 1], lane i.  Creating them takes about 0.4 ms, which would be a sixth of a
 // small engine's set-up, so a destroyed engine's set goes back to a process-wide pool
 // (at most kPooledLaneSets kept; mutex) and the next engine takes it.
 struct LaneSet {
+  cudaStream_t main = nullptr;        // the engine's own stream
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> ev;        // [0] fork, [i] end of side[i - 1]
+  cudaEvent_t t0 = nullptr, t1 = nullptr;  // timed builds
 };
 constexpr int kLanes = 8;
 constexpr size_t kPooledLaneSets = 4;
@@ -100,10 +102,12 @@ struct PairClassHost {
   std::vector<double> prim;        // SoA [PF_COUNT][Kab][n]
   int n() const { return (int)sa.size(); }
   // device copies
-  DevBuf d_sa, d_sb, d_fa, d_fb, d_Q, d_AB, d_Acen, d_prim, d_sys, d_primf, d_primb, d_primbf, d_primk,
-      d_primkf;
-  bool batched = false;             // d_sys is set (more than one system)
+  DevBuf d_sa, d_sb, d_fa, d_fb, d_Q, d_AB, d_Acen, d_prim, d_primb, d_primbf, d_primk, d_primkf;
+  bool batched = false;             // more than one system
+  bool on_device = false;           // an engine's class: its tables are in the engine's d_pairs
+  lai::PairClassDev dev{};
   lai::PairClassDev view() const {
+    if (on_device) return dev;
     lai::PairClassDev v;
     v.la = la; v.lb = lb; v.Ka = Ka; v.Kb = Kb; v.npairs = n();
     v.shell_a = d_sa.as<int>(); v.shell_b = d_sb.as<int>();
@@ -111,8 +115,8 @@ struct PairClassHost {
     v.Q = d_Q.as<double>(); v.AB = d_AB.as<double>(); v.Acen = d_Acen.as<double>();
     v.prim = d_prim.as<double>();
     v.qprim_max = qprim_max;
-    v.sys = batched ? d_sys.as<int>() : nullptr;
-    v.primf = d_primf.as<float>();
+    v.sys = nullptr;
+    v.primf = nullptr;
     v.primb = d_primb.as<double>();
     v.primbf = d_primbf.as<float>();
     v.primk = d_primk.as<double>();
@@ -124,9 +128,9 @@ struct PairClassHost {
 struct ClassPairBlock {
   int bra, ket;                 // class indices, bra >= ket
   std::vector<int64_t> offsets; // host copy
-  DevBuf d_offsets;
+  const int64_t* dev_offsets = nullptr;
   std::vector<int> qbegin;      // first ket of each bra pair (batched engines: its system's segment)
-  DevBuf d_qbegin;              // empty for a single system (every ket range starts at 0)
+  const int* dev_qbegin = nullptr;  // null for a single system (every ket range starts at 0)
   int64_t total = 0;
   double alg_flops = 0;         // per quartet of this block (all nonzero primitives)
   double flops_per_prim = 0;    // per primitive quartet
@@ -159,8 +163,8 @@ struct lai_engine {
   double thr = 1e-12;
   double prim_eps = 1e-15;
   cudaStream_t stream = nullptr;
-  lai::host::DevBuf d_coef, d_hx2, d_hw, d_boys, d_boys_f32, d_rys_f32;
   lai::RysTablesView tab{};
+  lai::host::DevBuf d_pairs;     // pair tables of every class and quartet ranges of every block
   std::vector<std::unique_ptr<lai::host::PairClassHost>> classes;
   std::vector<std::unique_ptr<lai::host::ClassPairBlock>> blocks;
   std::vector<double> Q_all;     // nshell x nshell Schwarz matrix
@@ -216,10 +220,7 @@ inline lai_engine::~lai_engine() {
   for (auto e : prof_ev) cudaEventDestroy(e);
   classes.clear();
   blocks.clear();
-  if (ev0) cudaEventDestroy(ev0);
-  if (ev1) cudaEventDestroy(ev1);
   lai::host::release_lanes(lanes);
-  if (stream) cudaStreamDestroy(stream);
 }
 
 namespace lai {
@@ -256,6 +257,13 @@ class LaunchLanes {
   std::vector<double> load_;   // estimated work per lane; < 0: not forked yet
 };
 double alg_work(int la, int lb, int lc, int ld, int Ka, int Kb, int Kc, int Kd);
+double alg_per_prim(int la, int lb, int lc, int ld);
+double alg_per_quartet(int la, int lb, int lc, int ld);
+
+// Implemented in setup.cu: the lookup tables, and the pair tables, bounds and quartet
+// ranges of the engine's classes (build_classes has listed their pairs).
+int setup_tables(lai_engine* E);
+int setup_pairs(lai_engine* E);
 
 }  // namespace host
 }  // namespace lai
