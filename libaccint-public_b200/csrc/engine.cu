@@ -293,7 +293,7 @@ int upload_class(PairClassHost& c) {
     const int n = c.n(), Kab = c.Ka * c.Kb;
     std::vector<double> rb((size_t)n * Kab * lai::kBraRec, 0.0);
     static const int from[lai::kBraRec] = {lai::PF_Q,  lai::PF_ZETA, lai::PF_HZ,  lai::PF_C,
-                                           lai::PF_PX, lai::PF_PY,   lai::PF_PZ,  -1,
+                                           lai::PF_PX, lai::PF_PY,   lai::PF_PZ,  lai::PF_ALPHA,
                                            lai::PF_PAX, lai::PF_PAY, lai::PF_PAZ, -1};
     for (int p = 0; p < n; ++p)
       for (int t = 0; t < Kab; ++t)
@@ -381,7 +381,7 @@ void release_lanes(LaneSet& set) {
   set = LaneSet{};
 }
 
-LaunchLanes::LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread) : E_(E), main_(stream), load_(1, 0.0) {
+LaunchLanes::LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread) : E_(E), main_(stream), load_(1, 0.0), lock_(E->lanes_mutex) {
   E->fork_stream = stream;
   if (!spread || E->lanes.side.empty()) return;
   if (cudaEventRecord(E->lanes.ev[0], stream) != cudaSuccess) return;  // one lane: the caller's stream
@@ -410,7 +410,10 @@ cudaError_t LaunchLanes::join() {
     if (e != cudaSuccess) rc = e;
   }
   load_.assign(1, 0.0);
-  E_->fork_stream = nullptr;
+  if (lock_.owns_lock()) {
+    E_->fork_stream = nullptr;
+    lock_.unlock();
+  }
   return rc;
 }
 

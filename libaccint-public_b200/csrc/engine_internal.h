@@ -7,6 +7,7 @@
 
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -211,6 +212,7 @@ struct lai_engine {
   int prof_n = 0;
   // streams the independent class-pair launches of one build are spread over
   lai::host::LaneSet lanes;
+  std::recursive_mutex lanes_mutex;   // held while launches are queued on the lanes
   cudaStream_t fork_stream = nullptr; // caller's stream while a build is spread over lanes
   std::vector<int> launch_order;      // blocks by descending estimated work
 };
@@ -248,6 +250,7 @@ class LaunchLanes {
  public:
   LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread);
   ~LaunchLanes() { join(); }
+  LaunchLanes(const LaunchLanes&) = delete;
   cudaError_t pick(double work, cudaStream_t* s);
   cudaError_t join();
 
@@ -255,6 +258,9 @@ class LaunchLanes {
   lai_engine* E_;
   cudaStream_t main_;
   std::vector<double> load_;   // estimated work per lane; < 0: not forked yet
+  // calls of several threads on one engine queue their launches one after another (they
+  // share the lanes' events)
+  std::unique_lock<std::recursive_mutex> lock_;
 };
 double alg_work(int la, int lb, int lc, int ld, int Ka, int Kb, int Kc, int Kd);
 double alg_per_prim(int la, int lb, int lc, int ld);

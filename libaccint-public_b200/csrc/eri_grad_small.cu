@@ -32,10 +32,10 @@ Launcher find(int la, int lb, int lc, int ld) {
 bool grad_small_supported(int la, int lb, int lc, int ld) { return grad_small::find(la, lb, lc, ld) != nullptr; }
 
 int launch_grad_small(const QuartetBlock& blk, const double* D, int nbf, const int* shell_atom, double* grad,
-                      double prim_eps, const RysTablesView& tab, cudaStream_t stream, int num_sms) {
+                      int grad_stride, double prim_eps, const RysTablesView& tab, cudaStream_t stream, int num_sms) {
   const auto f = grad_small::find(blk.bra.la, blk.bra.lb, blk.ket.la, blk.ket.lb);
   if (!f) return -1;
-  grad_small::GradSmallArgs ga{D, nbf, shell_atom, grad, prim_eps};
+  grad_small::GradSmallArgs ga{D, nbf, shell_atom, grad, grad_stride, prim_eps, 1};
   return f(blk, ga, tab, stream, num_sms);
 }
 

@@ -51,8 +51,10 @@ struct GradSmallArgs {
   const double* D;
   int nbf;
   const int* shell_atom;
-  double* grad;
+  double* grad;        // kGradCopies accumulators of grad_stride doubles each
+  int grad_stride;
   double prim_eps;
+  int ps;              // lanes per quartet (a power of two)
 };
 
 // Sum over the horizontal-transfer terms of one side: (a b| = sum_{k <= b}
@@ -128,19 +130,25 @@ __global__ void __launch_bounds__(128) grad_small_kernel(QuartetBlock blk, GradS
   // warps take chunks of 32 consecutive quartets (grid-stride); one bra search per
   // chunk, then each lane steps forward to its own bra pair (usually the same)
   const int lane = threadIdx.x & 31;
+  // ps lanes share a quartet: lane sub of the group takes bra primitive pairs sub,
+  // sub + ps, ...; blocks, transfer and contraction are linear in the primitive sum, so
+  // every lane contracts its part and only the derivatives are summed over the group
+  const int ps = ga.ps, qpw = 32 / ps, slot = lane / ps, sub = lane & (ps - 1);
   const int64_t nq = blk.total - blk.t_begin;
-  const int64_t nchunks = (nq + 31) / 32;
+  const int64_t nchunks = (nq + qpw - 1) / qpw;
   const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  double* const grad = ga.grad + (size_t)(wid % kGradCopies) * ga.grad_stride;
   for (int64_t ch = wid; ch < nchunks; ch += nw) {
-    const int64_t t0 = blk.t_begin + ch * 32;
-    const int64_t t = t0 + lane;
+    const int64_t t0 = blk.t_begin + ch * qpw;
+    const bool active = t0 + slot < blk.total;
+    const int64_t t = active ? t0 + slot : blk.total - 1;
     int pw = 0;
     if (lane == 0) pw = find_bra(blk.offsets, nbra, t0);
     pw = __shfl_sync(0xffffffffu, pw, 0);
-    if (t >= blk.total) continue;
     int p = pw;
     while (t >= __ldg(blk.offsets + p + 1)) ++p;
+    const bool uniform = __all_sync(0xffffffffu, p == pw);
     const int q = (blk.qbegin ? __ldg(blk.qbegin + p) : 0) + (int)(t - __ldg(blk.offsets + p));
     const double* __restrict__ pkt = ket_tile_ptr(blk.ket.primk, q, Kcd);
     double W[NWE * NWF], W2[AB_ ? NW2E * NWF : 1], W3[NW3E * NW3F], U[NUE * NUF];
@@ -153,7 +161,7 @@ __global__ void __launch_bounds__(128) grad_small_kernel(QuartetBlock blk, GradS
 #pragma unroll
     for (int i = 0; i < NUE * NUF; ++i) U[i] = 0.0;
 
-    for (int ib = 0; ib < Kab; ++ib) {
+    for (int ib = sub; ib < Kab; ib += ps) {
       // bra primitive: its per-pair record (the warp usually shares the bra pair);
       // the exponent on A from the SoA table
       const double2* rb = reinterpret_cast<const double2*>(blk.bra.primb + ((size_t)p * Kab + ib) * kBraRec);
@@ -291,7 +299,7 @@ __global__ void __launch_bounds__(128) grad_small_kernel(QuartetBlock blk, GradS
     }
     const int fa = __ldg(blk.bra.func_a + p), fb = __ldg(blk.bra.func_b + p);
     const int fc = __ldg(blk.ket.func_a + q), fd = __ldg(blk.ket.func_b + q);
-    const double s = quartet_weight(blk, p, q);
+    const double s = active ? quartet_weight(blk, p, q) : 0.0;
     const double* __restrict__ D = ga.D;
     const size_t nbf = (size_t)ga.nbf;
     double g[3] = {0.0, 0.0, 0.0}, g2[3] = {0.0, 0.0, 0.0};  // g2: the B centre of a merged pass
@@ -389,30 +397,37 @@ __global__ void __launch_bounds__(128) grad_small_kernel(QuartetBlock blk, GradS
         });
       });
     });
+    // sums over the quartet's lanes; then the centres of a bra pair that the whole warp
+    // shares go out once per warp, the others once per quartet
+    const int atC = __ldg(ga.shell_atom + __ldg(blk.ket.shell_a + q));
+    const int atD = __ldg(ga.shell_atom + __ldg(blk.ket.shell_b + q));
+    auto add = [&](int at, const double (&v)[3], bool of_bra) {
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        if (of_bra && uniform) {
+          double w = v[x];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+          if (lane == 0) atomicAdd(grad + 3 * at + x, w);
+        } else {
+          double w = v[x];
+          for (int o = ps >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+          if (active && sub == 0) atomicAdd(grad + 3 * at + x, w);
+        }
+      }
+    };
     const int sh = D1 == DA ? __ldg(blk.bra.shell_a + p) : D1 == DB ? __ldg(blk.bra.shell_b + p)
                                                                     : __ldg(blk.ket.shell_a + q);
-    const int at = __ldg(ga.shell_atom + sh);
-    const int atD = __ldg(ga.shell_atom + __ldg(blk.ket.shell_b + q));
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-      atomicAdd(ga.grad + 3 * at + x, g[x]);
-      atomicAdd(ga.grad + 3 * atD + x, -(g[x] + g2[x] + g3[x]));
-    }
-    if constexpr (AB_) {
-      const int atB = __ldg(ga.shell_atom + __ldg(blk.bra.shell_b + p));
-#pragma unroll
-      for (int x = 0; x < 3; ++x) atomicAdd(ga.grad + 3 * atB + x, g2[x]);
-    }
-    if constexpr (ABC_) {
-      const int atC = __ldg(ga.shell_atom + __ldg(blk.ket.shell_a + q));
-#pragma unroll
-      for (int x = 0; x < 3; ++x) atomicAdd(ga.grad + 3 * atC + x, g3[x]);
-    }
+    add(__ldg(ga.shell_atom + sh), g, D1 != DC);
+    if constexpr (AB_) add(__ldg(ga.shell_atom + __ldg(blk.bra.shell_b + p)), g2, true);
+    if constexpr (ABC_) add(atC, g3, false);
+    const double gd[3] = {-(g[0] + g2[0] + g3[0]), -(g[1] + g2[1] + g3[1]), -(g[2] + g2[2] + g3[2])};
+    add(atD, gd, false);
   }
 }
 
 template <int LA, int LB, int LC, int LD>
-int launch(const QuartetBlock& blk, const GradSmallArgs& ga, const RysTablesView& tab, cudaStream_t stream,
+int launch(const QuartetBlock& blk, const GradSmallArgs& ga_in, const RysTablesView& tab, cudaStream_t stream,
            int num_sms) {
   const int64_t nq = blk.total - blk.t_begin;
   if (nq <= 0) return 0;
@@ -457,7 +472,14 @@ int launch(const QuartetBlock& blk, const GradSmallArgs& ga, const RysTablesView
     attr = true;
   }
   const int threads = 128;
-  const int64_t want = (nq + threads - 1) / threads;
+  // lanes per quartet: as many as it takes to fill the device, at most one per bra
+  // primitive pair.  (H2O)6/cc-pVDZ, one lane each: the (ss|ss) launches of 1e3 - 1e4
+  // quartets with up to 6561 primitive quartets ran 0.3 - 0.5 ms each on a few warps.
+  const int Kab = blk.bra.Ka * blk.bra.Kb;
+  GradSmallArgs ga = ga_in;
+  ga.ps = 1;
+  while (ga.ps < 32 && ga.ps < Kab && nq * ga.ps < (int64_t)num_sms * 512) ga.ps <<= 1;
+  const int64_t want = (nq * ga.ps + threads - 1) / threads;
   const int grid = (int)(want < (int64_t)num_sms * 8 ? want : (int64_t)num_sms * 8);
   if constexpr (kAll) {
     grad_small_kernel<LA, LB, LC, LD, DABC><<<grid, threads, smem, stream>>>(blk, ga, tab);

@@ -52,16 +52,17 @@ int launch_generic(const QuartetBlock& blk, const JKArgs& args, const RysTablesV
 // its (e0|f0) block does not fit in shared memory; 0 if it fits.
 size_t generic_global_scratch_doubles(int la, int lb, int lc, int ld, int num_sms);
 
-// Nuclear-gradient kernel (eri_grad.cu): adds dE/dR of the block's quartets to
-// grad[natom][3] (E = 1/2 tr DJ - 1/4 tr DK at fixed D).  0 on success.
-int launch_grad(const QuartetBlock& blk, const double* D, int nbf, const int* shell_atom, double* grad,
-                double prim_eps, const RysTablesView& tab, cudaStream_t stream, double* gscratch,
-                size_t gscratch_doubles, int num_sms);
-size_t grad_global_scratch_doubles(int la, int lb, int lc, int ld, int num_sms);
+// Block-per-quartet gradient kernel (eri_grad_block.cu), any class: adds dE/dR of the block's quartets
+// (E = 1/2 tr DJ - 1/4 tr DK at fixed D) to grad.  0 on success.  grad holds kGradCopies
+// accumulators [natom][3], grad_stride doubles apart, that the caller sums: a gradient has
+// so few elements that the atomics of a whole launch would queue up on them.
+constexpr int kGradCopies = 64;
+int launch_grad_block(const QuartetBlock& blk, const double* D, int nbf, const int* shell_atom, double* grad,
+                      int grad_stride, double prim_eps, const RysTablesView& tab, cudaStream_t stream, int num_sms);
 // Thread-per-quartet gradient kernels for the low classes (eri_grad_small.cu): 0 when
-// launched, -1 when the class is not covered (use launch_grad), -3 on a CUDA error.
+// launched, -1 when the class is not covered (use launch_grad_block), -3 on a CUDA error.
 int launch_grad_small(const QuartetBlock& blk, const double* D, int nbf, const int* shell_atom, double* grad,
-                      double prim_eps, const RysTablesView& tab, cudaStream_t stream, int num_sms);
+                      int grad_stride, double prim_eps, const RysTablesView& tab, cudaStream_t stream, int num_sms);
 bool grad_small_supported(int la, int lb, int lc, int ld);
 
 }  // namespace lai

@@ -30,6 +30,22 @@ int ensure_atoms(lai_engine* E) {
   return LAI_OK;
 }
 
+// grad[i] = sum over the kGradCopies accumulators, stride doubles apart
+__global__ void sum_copies_kernel(const double* __restrict__ copies, int stride, int n, double* __restrict__ grad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+  for (int c = 0; c < lai::kGradCopies; ++c) s += copies[(size_t)c * stride + i];
+  grad[i] = s;
+}
+
+// Stream-ordered scratch of one call (calls of several threads or streams do not share it).
+struct StreamBuf {
+  void* p = nullptr;
+  cudaStream_t s = nullptr;
+  ~StreamBuf() { if (p) cudaFreeAsync(p, s); }
+};
+
 }  // namespace
 
 extern "C" {
@@ -47,7 +63,13 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
   LAI_CUDA_TRY(cudaSetDevice(engine->device));
   if (int rc = ensure_atoms(engine)) return rc;
   cudaStream_t stream_of_call = static_cast<cudaStream_t>(stream);
-  LAI_CUDA_TRY(cudaMemsetAsync(d_grad, 0, sizeof(double) * 3 * engine->natom, stream_of_call));
+  const int n3 = 3 * engine->natom, stride = (n3 + 15) / 16 * 16;
+  const size_t bytes = sizeof(double) * stride * lai::kGradCopies;
+  StreamBuf copies;
+  copies.s = stream_of_call;
+  LAI_CUDA_TRY(cudaMallocAsync(&copies.p, bytes, stream_of_call));
+  double* const acc = static_cast<double*>(copies.p);
+  LAI_CUDA_TRY(cudaMemsetAsync(acc, 0, bytes, stream_of_call));
   const int nbf = (int)engine->basis->nbf;
   LaunchLanes lanes(engine, stream_of_call, true);
   for (const int b : engine->launch_order) {
@@ -55,22 +77,19 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
     const lai::QuartetBlock q = make_block(engine, *bp);
     cudaStream_t s = stream_of_call;
     LAI_CUDA_TRY(lanes.pick(bp->alg_flops * (double)bp->total, &s));
-    const int rs = lai::launch_grad_small(q, d_D, nbf, engine->d_shell_atom.as<int>(), d_grad, engine->prim_eps,
+    const int rs = lai::launch_grad_small(q, d_D, nbf, engine->d_shell_atom.as<int>(), acc, stride, engine->prim_eps,
                                           engine->tab, s, engine->num_sms);
     if (rs == 0) continue;
     if (rs != -1)
       return fail(LAI_ECUDA, std::string("gradient launch failed: ") + cudaGetErrorString(cudaGetLastError()));
-    const size_t need = lai::grad_global_scratch_doubles(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb,
-                                                         engine->num_sms);
-    if (int rc = ensure_scratch(engine, need)) return rc;
-    if (need) s = stream_of_call;  // one scratch buffer: its users follow one another
-    const int rc = lai::launch_grad(q, d_D, nbf, engine->d_shell_atom.as<int>(), d_grad, engine->prim_eps,
-                                    engine->tab, s, engine->d_scratch.as<double>(), engine->scratch_doubles,
-                                    engine->num_sms);
+    const int rc = lai::launch_grad_block(q, d_D, nbf, engine->d_shell_atom.as<int>(), acc, stride, engine->prim_eps,
+                                          engine->tab, s, engine->num_sms);
     if (rc < 0)
       return fail(LAI_ECUDA, std::string("gradient launch failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
   LAI_CUDA_TRY(lanes.join());
+  if (n3 > 0) sum_copies_kernel<<<(n3 + 127) / 128, 128, 0, stream_of_call>>>(acc, stride, n3, d_grad);
+  LAI_CUDA_TRY(cudaGetLastError());
   return LAI_OK;
 }
 

@@ -48,8 +48,8 @@ enum PrimField : int {
 // and primitive) and each record is read with 16-byte vector loads.
 enum BraRecField : int {
   BR_Q = 0, BR_ZETA, BR_HZ, BR_C,   // first 16 bytes (FP32) / first two double2 (FP64)
-  BR_PX, BR_PY, BR_PZ, BR_PAD0,
-  BR_PAX, BR_PAY, BR_PAZ, BR_PAD1,
+  BR_PX, BR_PY, BR_PZ, BR_ALPHA,    // BR_ALPHA: exponent on the pair's first shell (gradients)
+  BR_PAX, BR_PAY, BR_PAZ, BR_PAD,
   kBraRec
 };
 

@@ -96,7 +96,7 @@ __global__ void build_tables_kernel(const ClassTables* __restrict__ cls, int ncl
   for (int k = 0; k < PF_COUNT; ++k) prim[k * sf + at] = f[k];
   double* rb = const_cast<double*>(o.primb) + ((size_t)p * c.Kab + t) * kBraRec;
   const double rec[kBraRec] = {f[PF_Q],  f[PF_ZETA], f[PF_HZ], f[PF_C], f[PF_PX], f[PF_PY],
-                               f[PF_PZ], 0.0,        f[PF_PAX], f[PF_PAY], f[PF_PAZ], 0.0};
+                               f[PF_PZ], f[PF_ALPHA], f[PF_PAX], f[PF_PAY], f[PF_PAZ], 0.0};
   for (int k = 0; k < kBraRec; ++k) rb[k] = rec[k];
   const double ket[kKetRec] = {f[PF_Q],   f[PF_ZETA], f[PF_HZ],  f[PF_PX], f[PF_PY], f[PF_PZ],
                                f[PF_PAX], f[PF_PAY],  f[PF_PAZ], f[PF_C],  f[PF_ALPHA]};
