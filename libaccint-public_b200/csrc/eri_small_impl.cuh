@@ -67,6 +67,38 @@ template <int LA, int LB, int LC, int LD, typename GV>
 __device__ __forceinline__ void small_finish(GV&& gval, const QuartetBlock& blk, const JKArgs& args,
                                              int64_t t, int p, int q, bool active, bool uniform_bra);
 
+// The FP64 classes of total angular momentum 2 and 3 with at most a p function on the ket
+// form (e0|f0) by the vertical recurrence over F_0..F_L instead of by Rys quadrature: a
+// Boys row is 5 16-byte shared-memory loads where the two-root fit is 24 (each lane on its
+// own row, so a warp's load is 4 to 10 shared-memory cycles; the FP64 work of a primitive
+// quartet is about 60 to 120 cycles), and the recurrence has fewer products than two sets
+// of 2-D tables.  (H2O)64/cc-pVDZ, Rys -> recurrence: (ps|ps) 234 -> 183 ms, (pp|ss) 104 ->
+// 78, (ds|ss) 85.5 -> 69.4, (pp|ps) 120 -> 109, (ds|ps) 108 -> 96, (dp|ss) 33.0 -> 30.5.
+template <int LA, int LB, int LC, int LD, typename R>
+__host__ __device__ constexpr bool small_vrr() {
+  return sizeof(R) == 8 && LA + LB + LC + LD >= 2 && LA + LB + LC + LD <= 3 && LC + LD <= 1;
+}
+// Whether the ket loop loads a primitive one iteration ahead.  Not in (ds|ps): without the
+// second copy it fits 128 registers and two blocks ((H2O)64/cc-pVDZ 99.7 -> 95.8 ms); the
+// other classes of the vertical recurrence lose 5 - 25 % without the prefetch.
+template <int LA, int LB, int LC, int LD, typename R>
+__host__ __device__ constexpr bool small_prefetch() {
+  return !(sizeof(R) == 8 && LA == 2 && LB == 0 && LC == 1 && LD == 0);
+}
+// Shared-memory table of a class: Boys rows (one root, or the vertical recurrence), the
+// Rys fits of its root count, or their FP32 versions.
+template <int LA, int LB, int LC, int LD, typename R>
+__host__ __device__ constexpr bool small_boys() {
+  return sizeof(R) == 8 && (LA + LB + LC + LD <= 1 || small_vrr<LA, LB, LC, LD, R>());
+}
+template <int LA, int LB, int LC, int LD, typename R>
+__host__ __device__ constexpr size_t small_table_bytes() {
+  constexpr int L = LA + LB + LC + LD;
+  if constexpr (sizeof(R) == 4) return f32_table_bytes<L / 2 + 1>();
+  else if constexpr (small_boys<LA, LB, LC, LD, R>()) return boys_rows_bytes<L>();
+  else return table_bytes<L / 2 + 1, double>();
+}
+
 template <int LA, int LB, int LC, int LD, typename R, bool SPLIT>
 __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKArgs& args,
                                               const RysTablesView& tab,
@@ -88,6 +120,8 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
   const size_t sb = (size_t)Kab * nbra;
 
   constexpr bool F32 = sizeof(R) == 4;
+  constexpr bool kVrr = small_vrr<LA, LB, LC, LD, R>();
+  constexpr int kL = LAB + LCD;
   // FP32: the primitive terms of one inner loop are summed in G, which is then
   // added to the running total Gc with a compensated (two-sum) step (registers
   // permitting: up to 18 (e0|f0) values); FP64: G is the total.
@@ -209,8 +243,15 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
       // One root: (ss|ss) = pref F_0 and (p_i s|ss) = pref (PA_i F_0 - rz PQ_i F_1)
       // -- the one-point Rys rule (w = F_0, u = F_1/F_0) written without its
       // quotient -- summed per row (fold_row) without the row's constant factor.
-      R F0, F1;
-      if constexpr (F32) boys01_f32(T, stab, F0, F1); else boys01_smem<R>(T, stab, F0, F1);
+      R F0, F1 = R(0);
+      if constexpr (F32) {
+        boys01_f32(T, stab, F0, F1);
+      } else {
+        double F[LAB + 1];
+        boys_rows<LAB>(T, stab, F);
+        F0 = F[0];
+        if constexpr (LAB == 1) F1 = F[1];
+      }
       static_assert(LAB == 0 || (LA == 1 && LB == 0 && LCD == 0), "one-root classes: (ss|ss), (ps|ss)");
       if constexpr (kFold) {
         const R pv = (kKetOuter ? cab : ccd) * rs;
@@ -232,6 +273,57 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
       return;
     }
     const R pref = cab * ccd * rs;
+    if constexpr (kVrr) {
+      // (e0|f0)^(m) by the vertical recurrence over Boys functions, e in LA..LAB and f in
+      // LC..LCD (LCD <= 1): V[e+1x]^(m) = PA_x V[e]^(m) - rz PQ_x V[e]^(m+1)
+      //   + e_x/(2 zeta) (V[e-1x]^(m) - rz V[e-1x]^(m+1)), and for f = p_x
+      //   V[e|p_x] = QC_x V[e]^(0) + re PQ_x V[e]^(1) + e_x/(2 (zeta+eta)) V[e-1x]^(1).
+      double F[kL + 1];
+      boys_rows<kL>(T, stab, F);
+      const double PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz};
+      const double WP[3] = {-rz * PQx, -rz * PQy, -rz * PQz}, WQ[3] = {re * PQx, re * PQy, re * PQz};
+      double V[kL + 1][LAB + 1][ncart(LAB)];  // [m][l][component]
+#pragma unroll
+      for (int m = 0; m <= kL; ++m) V[m][0][0] = pref * F[m];
+      sfor<1, LAB + 1>([&](auto LL) {
+        constexpr int l = decltype(LL)::value;
+        sfor<0, ncart(l)>([&](auto IE) {
+          constexpr int ie = decltype(IE)::value, c = cart_comp(l, ie);
+          constexpr int d = comp_x(c) ? 0 : comp_y(c) ? 1 : 2;  // direction lowered
+          constexpr int x = comp_x(c) - (d == 0), y = comp_y(c) - (d == 1), z = comp_z(c) - (d == 2);
+          constexpr int i1 = cart_index(x, y, z), nd = d == 0 ? x : d == 1 ? y : z;
+#pragma unroll
+          for (int m = 0; m <= kL - l; ++m) {
+            double v = PA[d] * V[m][l - 1][i1] + WP[d] * V[m + 1][l - 1][i1];
+            if constexpr (nd > 0) {
+              constexpr int i2 = cart_index(x - (d == 0), y - (d == 1), z - (d == 2));
+              v += nd * hz * (V[m][l >= 2 ? l - 2 : 0][i2] - rz * V[m + 1][l >= 2 ? l - 2 : 0][i2]);
+            }
+            V[m][l][ie] = v;
+          }
+        });
+      });
+      sfor<0, NE>([&](auto IE) {
+        constexpr int ie = decltype(IE)::value;
+        constexpr int le = [] { int l = LA, r = ie; while (r >= ncart(l)) { r -= ncart(l); ++l; } return l; }();
+        constexpr int ic = ie - ncart_before(LA, le), ce = cart_comp(le, ic);
+        if constexpr (LC == 0) G[ie * NF] += V[0][le][ic];
+        if constexpr (LCD == 1) {
+          constexpr int f0 = LC == 0 ? 1 : 0;
+          sfor<0, 3>([&](auto XX) {
+            constexpr int x = decltype(XX)::value;
+            constexpr int ex = x == 0 ? comp_x(ce) : x == 1 ? comp_y(ce) : comp_z(ce);
+            double g = G[ie * NF + f0 + x] + QC[x] * V[0][le][ic] + WQ[x] * V[1][le][ic];
+            if constexpr (ex > 0) {
+              constexpr int i1 = cart_index(comp_x(ce) - (x == 0), comp_y(ce) - (x == 1), comp_z(ce) - (x == 2));
+              g += (0.5 * ex) * inv * V[1][le >= 1 ? le - 1 : 0][i1];
+            }
+            G[ie * NF + f0 + x] = g;
+          });
+        }
+      });
+      return;
+    }
     R u[NR], w[NR];
     if constexpr (F32) rys_f32(NR, T, stab, tab.herm_x2, tab.herm_w, u, w);
     else rys_smem<NR, R>(T, stab, tab, u, w);
@@ -312,8 +404,9 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
   } else {
     const R qket_max = R(blk.ket.qprim_max);
     // the first ket primitive opens every row: loaded once per quartet
+    constexpr bool kAhead = small_prefetch<LA, LB, LC, LD, R>();
     KetPrimT<R> k0;
-    load_ket_rec(pkt, k0);
+    if constexpr (kAhead) load_ket_rec(pkt, k0);
     for (int ib = ib0; ib < Kab; ib += ibs) {
       R qab;
       BraVals bv;
@@ -321,9 +414,11 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
       if (qab * qket_max < peps_r) break;
       KetPrimT<R> nxt = k0;
       for (int ik = 0; ik < Kcd; ++ik) {
+        if constexpr (!kAhead) load_ket_rec(pkt + (size_t)ik * kKetPrimStride, nxt);
         const KetPrimT<R> cur = nxt;
         if (qab * cur.q < peps_r) break;
-        if (ik + 1 < Kcd) load_ket_rec(pkt + (size_t)(ik + 1) * kKetPrimStride, nxt);
+        if constexpr (kAhead)
+          if (ik + 1 < Kcd) load_ket_rec(pkt + (size_t)(ik + 1) * kKetPrimStride, nxt);
         ++nprim_done;
         prim(bv, cur);
       }
@@ -602,7 +697,7 @@ __device__ __forceinline__ void small_finish(GV&& gval, const QuartetBlock& blk,
 // blocks, 32 warps; at 3 blocks it takes 72 without spilling and runs 1-2 % slower);
 // (ps|ss), with the first ket primitive held across its bra
 // rows, takes up to 128 without spilling (2 blocks; measured faster than 80
-// registers with spills at 3 blocks); in FP32 the one-root classes fit 64 and the
+// registers with spills at 3 blocks), and so do the L = 2 classes; in FP32 the one-root classes fit 64 and the
 // L = 2 ones, with their compensated accumulators, 128 (2 blocks).  FP64 (dp|ss)
 // and (fs|ss) fit 128 without spilling (left free, ptxas takes 178 for (dp|ss) and
 // the class runs 19 % slower on one block).  The other classes keep ptxas's own
@@ -612,7 +707,7 @@ __device__ __forceinline__ void small_finish(GV&& gval, const QuartetBlock& blk,
 template <int LA, int LB, int LC, int LD, typename R>
 __host__ __device__ constexpr int small_min_blocks() {
   constexpr int L = LA + LB + LC + LD;
-  return sizeof(R) == 8 ? (L == 0 ? 4 : L == 1 ? 2 : (LA + LB == 3 && LC + LD == 0) ? 2 : 0)
+  return sizeof(R) == 8 ? (L == 0 ? 4 : L <= 2 ? 2 : (LA + LB == 3 && LC + LD == 0) ? 2 : 0)
                         : (L <= 1 ? 4 : L == 2 ? 2 : 0);
 }
 
@@ -623,6 +718,7 @@ __global__ void __launch_bounds__(256, (small_min_blocks<LA, LB, LC, LD, R>()))
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* stab = reinterpret_cast<R*>(smem_raw);
   if constexpr (sizeof(R) == 4) stage_table_f32<NR>(reinterpret_cast<float*>(smem_raw), tab);
+  else if constexpr (small_boys<LA, LB, LC, LD, R>()) stage_boys_rows<LA + LB + LC + LD>(stab, tab);
   else stage_table<NR, R>(stab, tab);
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -667,9 +763,8 @@ namespace small_detail {
 template <int LA, int LB, int LC, int LD>
 int launch_one(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,
                cudaStream_t stream, bool fp32, int num_sms, LaunchTune tune) {
-  constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
   const int threads = 256;
-  const size_t smem = fp32 ? f32_table_bytes<NR>() : table_bytes<NR, double>();
+  const size_t smem = fp32 ? small_table_bytes<LA, LB, LC, LD, float>() : small_table_bytes<LA, LB, LC, LD, double>();
   const int64_t nq = blk.total - blk.t_begin;
   if (nq <= 0) return 1;
   // lanes per quartet: split the bra primitive loop when the launch has too few

@@ -123,6 +123,99 @@ __device__ __forceinline__ void boys01_smem(R T, const R* __restrict__ st, R& F0
   }
 }
 
+// Boys rows for F_0 .. F_L, L <= 3 (the thread-per-quartet kernels of the low classes).
+// Row k, of 10 doubles (five 16-byte units, odd, so lanes on different rows spread over
+// the banks), holds Taylor coefficients about T0 = k / 10, divided by j!:
+//   L = 0: F_j / j!, j < 8;  L = 1: F_j / j!, j < 9 (F_1 is the derivative of the same
+//   polynomial);  L >= 2: F_{L+j} / j!, j < 8, and exp(-T0), for the downward recursion
+//   F_{m-1} = (2 T F_m + exp(-T)) / (2m - 1).
+// The first omitted term is below 0.05^8/8!/17 = 6e-17.  Above the grid the asymptotic
+// forms hold to 1e-16 of F_L: from 39.95 (L <= 1), 45.95 (L = 2, 3; the rows past the
+// stored grid come from F_0 = sqrt(pi/T)/2 and the upward recursion).
+constexpr int kBoysRowLen = 10;
+template <int L>
+__host__ __device__ constexpr int boys_rows_n() { return L <= 1 ? kBoysNGrid : 461; }
+template <int L>
+__host__ __device__ constexpr double boys_rows_tmax() { return L <= 1 ? kBoysTmax : 45.95; }
+template <int L>
+__host__ __device__ constexpr size_t boys_rows_bytes() { return sizeof(double) * kBoysRowLen * boys_rows_n<L>(); }
+
+template <int L>
+__device__ __forceinline__ void stage_boys_rows(double* __restrict__ st, const RysTablesView& tab) {
+  constexpr int NV = L == 1 ? 9 : 8;
+  for (int k = threadIdx.x; k < boys_rows_n<L>(); k += blockDim.x) {
+    double* row = st + k * kBoysRowLen;
+    double F[L + 9];
+    const double T = k * 0.1, e = L >= 2 ? exp(-T) : 0.0;
+    if (k < kBoysNGrid) {
+#pragma unroll
+      for (int j = 0; j < L + 9; ++j) F[j] = __ldg(tab.boys + k * kBoysNM + j);
+    } else {
+      F[0] = 0.88622692545275801365 * rsqrt(T);
+#pragma unroll
+      for (int j = 0; j < L + 8; ++j) F[j + 1] = ((2 * j + 1) * F[j] - e) / (2.0 * T);
+    }
+    constexpr int m0 = L >= 2 ? L : 0;
+    double f = 1.0;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      row[j] = F[m0 + j] * f;
+      f /= j + 1;
+    }
+    if (L >= 2) row[8] = e;
+  }
+}
+
+template <int L>
+__device__ __forceinline__ void boys_rows(double T, const double* __restrict__ st, double (&F)[L + 1]) {
+  static_assert(L >= 0 && L <= 3, "F_0 .. F_3");
+  if (T < boys_rows_tmax<L>()) {
+    const double km = fma(T, 10.0, kRoundMagicD);  // nearest row (no conversion instructions)
+    const int k = min(__double2loint(km), boys_rows_n<L>() - 1);
+    const double x = fma(km - kRoundMagicD, 0.1, -T);
+    const double2* r = reinterpret_cast<const double2*>(st + k * kBoysRowLen);
+    double g[10];
+#pragma unroll
+    for (int j = 0; j < (L == 0 ? 4 : 5); ++j) {
+      const double2 v = r[j];
+      g[2 * j] = v.x;
+      g[2 * j + 1] = v.y;
+    }
+    if constexpr (L == 1) {
+      double a = fma(g[8], x, g[7]), d = g[8];  // polynomial and its derivative
+#pragma unroll
+      for (int j = 6; j >= 0; --j) {
+        d = fma(d, x, a);
+        a = fma(a, x, g[j]);
+      }
+      F[0] = a;
+      F[1] = d;
+    } else {
+      double a = g[7];
+#pragma unroll
+      for (int j = 6; j >= 0; --j) a = fma(a, x, g[j]);
+      F[L] = a;
+      if constexpr (L >= 2) {
+        // exp(-T) = exp(-T0) exp(x), |x| <= 0.05: degree 8 leaves 0.05^9/9! = 5e-18
+        constexpr double c[9] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320};
+        double ex = c[8];
+#pragma unroll
+        for (int j = 7; j >= 0; --j) ex = fma(ex, x, c[j]);
+        ex *= g[8];
+        const double t2 = T + T;
+#pragma unroll
+        for (int m = L; m >= 1; --m) F[m - 1] = fma(t2, F[m], ex) * (1.0 / (2 * m - 1));
+      }
+    }
+  } else {
+    const double rt = fast_rsqrt(T);
+    F[0] = 0.88622692545275801365 * rt;  // sqrt(pi)/2
+    const double h = 0.5 * rt * rt;
+#pragma unroll
+    for (int m = 1; m <= L; ++m) F[m] = (2 * m - 1) * h * F[m - 1];
+  }
+}
+
 // Roots/weights of the NR-point Rys rule from the staged table (same arithmetic
 // as rys_roots_table in rys_eval.h).
 template <int NR, typename R>
