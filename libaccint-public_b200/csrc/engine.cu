@@ -181,14 +181,21 @@ double alg_work(int la, int lb, int lc, int ld, int Ka, int Kb, int Kc, int Kd) 
   return P * alg_per_prim(la, lb, lc, ld) + alg_per_quartet(la, lb, lc, ld);
 }
 
+// J = J' + J'^T, K = K' + K'^T, J' and K' the sums of `copies` accumulators of n^2 elements.
 __global__ void symmetrize_kernel(const double* __restrict__ Jp, const double* __restrict__ Kp,
-                                  double* __restrict__ J, double* __restrict__ K, int n) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)n * n) return;
+                                  double* __restrict__ J, double* __restrict__ K, int n, int copies) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nn = (int64_t)n * n;
+  if (idx >= nn) return;
   const int i = (int)(idx / n), j = (int)(idx - (int64_t)i * n);
   const int64_t tr = (int64_t)j * n + i;
-  J[idx] = Jp[idx] + Jp[tr];
-  K[idx] = Kp[idx] + Kp[tr];
+  double sj = 0.0, sk = 0.0;
+#pragma unroll 4
+  for (int c = 0; c < copies; ++c, Jp += nn, Kp += nn) {
+    sj += Jp[idx] + Jp[tr];
+    sk += Kp[idx] + Kp[tr];
+  }
+  J[idx] = sj;
+  K[idx] = sk;
 }
 
 }  // namespace host
@@ -351,6 +358,21 @@ void destroy_lanes(LaneSet& set) {
 }
 }  // namespace
 
+// The first n - 1 side streams (and their events) of the set.
+int extend_lanes(LaneSet& set, size_t n) {
+  while (set.ev.size() < n) {
+    cudaEvent_t e = nullptr;
+    LAI_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    set.ev.push_back(e);
+  }
+  while (set.side.size() + 1 < n) {
+    cudaStream_t s = nullptr;
+    LAI_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    set.side.push_back(s);
+  }
+  return LAI_OK;
+}
+
 int acquire_lanes(LaneSet& out) {
   {
     std::lock_guard<std::mutex> lock(g_lane_mutex);
@@ -360,10 +382,7 @@ int acquire_lanes(LaneSet& out) {
       return LAI_OK;
     }
   }
-  out.side.assign(kLanes - 1, nullptr);
-  out.ev.assign(kLanes, nullptr);
-  for (auto& s : out.side) LAI_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  for (auto& e : out.ev) LAI_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (int rc = extend_lanes(out, kLanes)) return rc;
   LAI_CUDA_TRY(cudaStreamCreateWithFlags(&out.main, cudaStreamNonBlocking));
   LAI_CUDA_TRY(cudaEventCreate(&out.t0));
   LAI_CUDA_TRY(cudaEventCreate(&out.t1));
@@ -373,7 +392,7 @@ int acquire_lanes(LaneSet& out) {
 // Work still queued on the set's streams was joined to the caller's stream, and the next
 // engine's work on them simply follows it.
 void release_lanes(LaneSet& set) {
-  if (set.side.size() != (size_t)kLanes - 1 || set.ev.size() != (size_t)kLanes || !set.t1)
+  if (set.side.size() + 1 < (size_t)kLanes || !set.t1)
     return destroy_lanes(set);
   std::lock_guard<std::mutex> lock(g_lane_mutex);
   if (lane_pool().size() >= kPooledLaneSets) return destroy_lanes(set);
@@ -381,11 +400,12 @@ void release_lanes(LaneSet& set) {
   set = LaneSet{};
 }
 
-LaunchLanes::LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread) : E_(E), main_(stream), load_(1, 0.0), lock_(E->lanes_mutex) {
+LaunchLanes::LaunchLanes(lai_engine* E, cudaStream_t stream, size_t lanes) : E_(E), main_(stream), load_(1, 0.0), lock_(E->lanes_mutex) {
   E->fork_stream = stream;
-  if (!spread || E->lanes.side.empty()) return;
+  lanes = std::min(lanes, E->lanes.side.size() + 1);
+  if (lanes < 2) return;
   if (cudaEventRecord(E->lanes.ev[0], stream) != cudaSuccess) return;  // one lane: the caller's stream
-  load_.resize(E->lanes.side.size() + 1, -1.0);
+  load_.resize(lanes, -1.0);
 }
 
 cudaError_t LaunchLanes::pick(double work, cudaStream_t* s) {
@@ -423,7 +443,9 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
                  bool fp32, bool* ran_fp32, lai::LaunchTune tune) {
   const int la = blk.bra.la, lb = blk.bra.lb, lc = blk.ket.la, ld = blk.ket.lb;
   if (ran_fp32) *ran_fp32 = false;
-  if (lai::small_class_supported(la, lb, lc, ld)) {
+  const bool untuned = tune.ps == 0 && tune.ksuper == 0 && tune.kernel == lai::KERNEL_DEFAULT;
+  if (untuned && !fp32 && args.mode == lai::MODE_JK && lai::block_for_few(blk, E->num_sms)) tune.kernel = lai::KERNEL_BLOCK;
+  if (lai::small_class_supported(la, lb, lc, ld) && tune.kernel != lai::KERNEL_BLOCK) {
     const int rc = lai::launch_small(blk, args, E->tab, E->stream, fp32, E->num_sms, tune);
     if (ran_fp32) *ran_fp32 = fp32;
     if (rc < 0) return fail(LAI_ECUDA, std::string("small-class launch failed: ") +
@@ -550,12 +572,27 @@ int build_split(lai_engine* E, double cut) {
   return LAI_OK;
 }
 
+// Accumulators of J' (and of K') in a build: four for the systems of some hundred
+// functions, whose elements collect thousands of additions each, in an order that the
+// concurrent launches change (run to run 1e-13 of the largest element with one).  Smaller
+// systems add too few, and larger ones spread their additions over more elements.
+int accumulator_copies(size_t elems) { return elems >= (size_t(1) << 15) && elems <= (size_t(1) << 19) ? 4 : 1; }
+
+// J' and K' of a build, elems each, one buffer (J' first).
+int ensure_accumulators(lai_engine* E, size_t elems) {
+  const size_t bytes = 2 * sizeof(double) * elems;
+  if (E->d_JKp.bytes >= bytes) return LAI_OK;
+  E->release_graph();
+  LAI_CUDA_TRY(E->d_JKp.alloc(bytes));
+  return LAI_OK;
+}
+
 // J = J' + J'^T, K = K' + K'^T on every system block of a batched engine's packed
 // matrices (block s = nbf_s x nbf_s at element offset off[s]).
 __global__ void symmetrize_batched_kernel(const double* __restrict__ Jp, const double* __restrict__ Kp,
                                           double* __restrict__ J, double* __restrict__ K,
                                           const int64_t* __restrict__ off, const int* __restrict__ nbfs,
-                                          int nsys) {
+                                          int nsys, int copies) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= off[nsys]) return;
   int lo = 0, hi = nsys;  // off[lo] <= idx < off[hi]
@@ -566,35 +603,146 @@ __global__ void symmetrize_batched_kernel(const double* __restrict__ Jp, const d
   const int n = nbfs[lo];
   const int64_t l = idx - off[lo];
   const int i = (int)(l / n), j = (int)(l - (int64_t)i * n);
-  const int64_t tr = off[lo] + (int64_t)j * n + i;
-  J[idx] = Jp[idx] + Jp[tr];
-  K[idx] = Kp[idx] + Kp[tr];
+  const int64_t tr = off[lo] + (int64_t)j * n + i, all = off[nsys];
+  double sj = 0.0, sk = 0.0;
+#pragma unroll 4
+  for (int c = 0; c < copies; ++c, Jp += all, Kp += all) {
+    sj += Jp[idx] + Jp[tr];
+    sk += Kp[idx] + Kp[tr];
+  }
+  J[idx] = sj;
+  K[idx] = sk;
 }
 
-// forced_cut >= 0: use this Schwarz cut for the FP32 split instead of deriving it
-// from max|D| (which synchronizes the stream; not allowed while capturing a graph).
-int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t stream,
-           const lai_jk_opts& o, lai_jk_report* rep, bool timed, double forced_cut = -1.0) {
+// The launches of a plain build.  An engine has a block per pair of classes (la, lb, Ka, Kb),
+// H2O/cc-pVQZ 666 of them for 120 angular classes; a launch each leaves the device to
+// their set-up (lookup tables, class tables, 15 - 25 us of latency whatever the work).
+// The blocks of one angular class that do not fill the device alone go out as one launch,
+// each with its own split of a quartet, the heaviest items first.
+int build_launches(lai_engine* E) {
+  const int nb = (int)E->blocks.size();
+  std::map<std::array<int, 5>, std::vector<int>> groups;  // kernel and class -> blocks
+  std::vector<int> single;
+  for (int b = 0; b < nb; ++b) {
+    const lai::QuartetBlock q = make_block(E, *E->blocks[b]);
+    const int la = q.bra.la, lb = q.bra.lb, lc = q.ket.la, ld = q.ket.lb;
+    int kind = 0;  // 1: thread-per-quartet, split; 2: block-per-quartet
+    if (lai::small_class_supported(la, lb, lc, ld))
+      kind = lai::block_for_few(q, E->num_sms) ? 2 : q.total < (int64_t)E->num_sms * lai::kSplitQuartetsPerSm ? 1 : 0;
+    else if (lai::default_kernel(la, lb, lc, ld, q.total, E->num_sms) == lai::KERNEL_BLOCK)
+      kind = 2;
+    if (kind) groups[{kind, la, lb, lc, ld}].push_back(b);
+    else single.push_back(b);
+  }
+  std::vector<lai::MultiEntry> entries;
+  auto work_of = [&](int b) { return E->blocks[b]->alg_flops * (double)E->blocks[b]->total; };
+  auto add_single = [&](int b) {
+    lai_engine::LaunchItem it;
+    it.block = b;
+    it.work = work_of(b);
+    E->launches.push_back(it);
+  };
+  for (int b : single) add_single(b);
+  for (auto& [key, blocks] : groups) {
+    if (blocks.size() == 1) {
+      add_single(blocks[0]);
+      continue;
+    }
+    lai_engine::LaunchItem it;
+    it.block_kernel = key[0] == 2;
+    it.la = key[1]; it.lb = key[2]; it.lc = key[3]; it.ld = key[4];
+    it.first = (int)entries.size();
+    it.n = (int)blocks.size();
+    double prims = 0.0;
+    std::vector<lai::MultiEntry> es;
+    std::vector<int64_t> P;
+    for (int b : blocks) {
+      lai::MultiEntry e{};
+      e.blk = make_block(E, *E->blocks[b]);
+      P.push_back((int64_t)e.blk.bra.Ka * e.blk.bra.Kb * e.blk.ket.Ka * e.blk.ket.Kb);
+      prims += (double)P.back() * (double)e.blk.total;
+      it.Pmax = std::max(it.Pmax, P.back());
+      it.work += work_of(b);
+      e.ps = e.nsplit = e.csplit = 1;
+      es.push_back(e);
+    }
+    if (!it.block_kernel) {
+      // lanes per quartet: no lane with more than a quarter of its share of the launch in
+      // one quartet (or 24 primitive quartets), and enough lanes to fill the device
+      const double lanes = 512.0 * E->num_sms, most = std::max(24.0, 0.25 * prims / lanes);
+      double used = 0.0;
+      for (size_t i = 0; i < es.size(); ++i) {
+        const int Kab = es[i].blk.bra.Ka * es[i].blk.bra.Kb;
+        while (es[i].ps < 32 && es[i].ps < Kab && (double)P[i] / es[i].ps > most) es[i].ps <<= 1;
+        es[i].nsplit = (int)std::max(1.0, std::min((double)(P[i] / Kab), (double)P[i] / es[i].ps / most));
+        used += (double)es[i].blk.total * es[i].ps;
+      }
+      for (bool grew = true; grew && used < lanes;) {
+        grew = false;
+        for (auto& e : es)
+          if (e.ps < 32 && e.ps < e.blk.bra.Ka * e.blk.bra.Kb) {
+            used += (double)e.blk.total * e.ps;
+            e.ps <<= 1;
+            grew = true;
+          }
+      }
+    } else {
+      // the same over blocks: four per SM, a quartet's primitive quartets first
+      const double slots = 4.0 * E->num_sms;
+      const int nroots = (it.la + it.lb + it.lc + it.ld) / 2 + 1;
+      const int rows = lai::ncart_range(it.la, it.la + it.lb);
+      const double least = 2.0 * std::max(1, (rows + 31) / 32 * 32 / (3 * nroots));
+      const double most = std::max(least, prims / (2.0 * slots));
+      double used = 0.0;
+      for (size_t i = 0; i < es.size(); ++i) {
+        es[i].nsplit = (int)std::max(1.0, std::min((double)P[i] / most, 1024.0));
+        used += (double)es[i].blk.total * es[i].nsplit;
+      }
+      const int nchunks = lai::block_ket_chunks(it.lc, it.ld);
+      const int cs = (int)std::max(1.0, std::min((double)nchunks, slots / used));
+      for (auto& e : es) e.csplit = cs;
+    }
+    // heaviest work items first
+    std::vector<int> order(es.size());
+    std::iota(order.begin(), order.end(), 0);
+    auto cost = [&](int i) { return (double)P[i] / es[i].nsplit / (it.block_kernel ? 1 : es[i].ps); };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
+    for (int i : order) {
+      lai::MultiEntry e = es[i];
+      e.work0 = it.nwork;
+      const int per = 32 / e.ps;
+      it.nwork += it.block_kernel ? e.blk.total * e.nsplit * e.csplit : (e.blk.total + per - 1) / per * e.nsplit;
+      entries.push_back(e);
+    }
+    E->launches.push_back(it);
+  }
+  std::stable_sort(E->launches.begin(), E->launches.end(),
+                   [](const auto& x, const auto& y) { return x.work > y.work; });
+  return upload(E->d_multi, entries) == cudaSuccess ? LAI_OK : fail(LAI_ECUDA, "launch list upload failed");
+}
+
+// J' = K' = 0 and every class-pair launch of a build of the density dD, on `stream`
+// (spread over the lanes).  Part 1 of a mixed build's blocks runs in FP32.
+int enqueue_jk(lai_engine* E, const double* dD, cudaStream_t stream, const lai_jk_opts& o, double cut, bool timed,
+               lai_jk_report& rep) {
   const int nbf = (int)E->basis->nbf;
   const bool batched = E->nsys > 1;
   const size_t elems = engine_mat_elems(E);
-  const size_t bytes = sizeof(double) * elems;
-  if (o.shard_count < 1 || o.shard_index < 0 || o.shard_index >= o.shard_count)
-    return fail(LAI_EINVAL, "lai_jk: bad shard_index/shard_count");
-  if (E->d_Jp.bytes < bytes) {
-    E->release_graph();
-    LAI_CUDA_TRY(E->d_Jp.alloc(bytes));
-    LAI_CUDA_TRY(E->d_Kp.alloc(bytes));
-  }
-  cudaStream_t saved = E->stream;
+  struct Restore {
+    lai_engine* E;
+    cudaStream_t saved;
+    ~Restore() { E->stream = saved; }
+  } restore{E, E->stream};
   E->stream = stream;
-  LAI_CUDA_TRY(cudaMemsetAsync(E->d_Jp.p, 0, bytes, stream));
-  LAI_CUDA_TRY(cudaMemsetAsync(E->d_Kp.p, 0, bytes, stream));
+  const int copies = accumulator_copies(elems);
+  LAI_CUDA_TRY(cudaMemsetAsync(E->d_JKp.p, 0, 2 * sizeof(double) * copies * elems, stream));
   if (timed) LAI_CUDA_TRY(cudaEventRecord(E->ev0, stream));
   lai::JKArgs args{};
   args.D = dD;
-  args.J = E->d_Jp.as<double>();
-  args.K = E->d_Kp.as<double>();
+  args.J = E->jp();
+  args.K = E->kp(copies * elems);
+  args.copy_mask = copies - 1;
+  args.copy_stride = (int64_t)elems;
   args.nbf = nbf;
   args.mode = lai::MODE_JK;
   args.prim_eps = E->prim_eps;
@@ -606,20 +754,7 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
   int launches = 0;
   int64_t nq = 0, nq32 = 0;
   double flops = 0;
-  // Mixed precision: a quartet runs in FP32 when Q_ij Q_kl max|D| < fp32_cut.  The
-  // Schwarz cut fp32_cut / max|D| is rounded down to a power of two (conservative:
-  // fewer FP32 quartets), so that the split, built on the host, is rebuilt only
-  // when max|D| moves past a power of two.
-  double cut = forced_cut >= 0.0 ? forced_cut : 0.0;
-  if (o.fp32_cut > 0.0 && forced_cut < 0.0) {
-    double maxd = 0.0;
-    if (int rc = device_absmax(E, dD, elems, stream, &maxd)) { E->stream = saved; return rc; }
-    if (maxd > 0.0 && std::isfinite(maxd)) cut = std::exp2(std::floor(std::log2(o.fp32_cut / maxd)));
-  }
   const bool mixed = cut > 0.0;
-  if (mixed) {
-    if (int rc = build_split(E, cut)) { E->stream = saved; return rc; }
-  }
   const int nparts = mixed ? 2 : 1;
   if (o.profile) {
     const size_t need = 2 * nparts * E->blocks.size();
@@ -637,7 +772,28 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
   }
   E->prof_n = 0;
   // profiled builds time every launch by itself, in block order on one stream
-  LaunchLanes lanes(E, stream, !o.profile);
+  LaunchLanes lanes(E, stream, o.profile ? 1 : kLanes);
+  if (!o.profile && !mixed && o.shard_count == 1 && !E->tuned) {
+    for (const auto& it : E->launches) {
+      LAI_CUDA_TRY(lanes.pick(it.work, &E->stream));
+      if (it.block >= 0) {
+        if (int rc = launch_block(E, make_block(E, *E->blocks[it.block]), args)) return rc;
+      } else {
+        const lai::MultiEntry* list = E->d_multi.as<lai::MultiEntry>() + it.first;
+        const int rc = it.block_kernel
+                           ? lai::launch_blockq_list(it.la, it.lb, it.lc, it.ld, it.Pmax, list, it.n, it.nwork, args,
+                                                     E->tab, E->stream, E->num_sms)
+                           : lai::launch_small_list(it.la, it.lb, it.lc, it.ld, list, it.n, it.nwork, args, E->tab,
+                                                    E->stream, E->num_sms);
+        if (rc < 0) return fail(LAI_ECUDA, std::string("launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+      }
+      ++launches;
+    }
+    for (const auto& b : E->blocks) {
+      nq += b->total;
+      flops += b->alg_flops * (double)b->total;
+    }
+  } else
   for (size_t i = 0; i < E->blocks.size(); ++i) {
     const size_t b = o.profile ? i : (size_t)E->launch_order[i];
     const auto& bp = *E->blocks[b];
@@ -660,11 +816,8 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
       args.prim_count = o.profile ? E->d_prof_prims.as<unsigned long long>() + E->prof_n : nullptr;
       if (o.profile) LAI_CUDA_TRY(cudaEventRecord(E->prof_ev[2 * E->prof_n], stream));
       bool ran32 = false;
-      if (cudaError_t ce = lanes.pick(bp.alg_flops * (double)(hi - lo), &E->stream)) {
-        E->stream = saved;
-        return fail(LAI_ECUDA, std::string("lai_jk: ") + cudaGetErrorString(ce));
-      }
-      if (int rc = launch_block(E, q, args, part == 1, &ran32, bp.tune)) { E->stream = saved; return rc; }
+      LAI_CUDA_TRY(lanes.pick(bp.alg_flops * (double)(hi - lo), &E->stream));
+      if (int rc = launch_block(E, q, args, part == 1, &ran32, bp.tune)) return rc;
       if (o.profile) {
         LAI_CUDA_TRY(cudaEventRecord(E->prof_ev[2 * E->prof_n + 1], stream));
         E->prof_block.push_back((int)b);
@@ -677,28 +830,57 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
       flops += bp.alg_flops * (double)(hi - lo);
     }
   }
-  E->stream = saved;
   LAI_CUDA_TRY(lanes.join());
+  rep.quartets_fp64 = nq - nq32;
+  rep.quartets_fp32 = nq32;
+  rep.fp32_schwarz_cut = cut;
+  rep.alg_flops = flops;
+  rep.kernel_launches = launches;
+  rep.seconds_device = 0;
+  return LAI_OK;
+}
+
+// forced_cut >= 0: use this Schwarz cut for the FP32 split instead of deriving it
+// from max|D| (which synchronizes the stream; not allowed while capturing a graph).
+int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t stream,
+           const lai_jk_opts& o, lai_jk_report* rep, bool timed, double forced_cut = -1.0) {
+  const int nbf = (int)E->basis->nbf;
+  const bool batched = E->nsys > 1;
+  const size_t elems = engine_mat_elems(E);
+  if (o.shard_count < 1 || o.shard_index < 0 || o.shard_index >= o.shard_count)
+    return fail(LAI_EINVAL, "lai_jk: bad shard_index/shard_count");
+  const int copies = accumulator_copies(elems);
+  if (int rc = ensure_accumulators(E, copies * elems)) return rc;
+  // Mixed precision: a quartet runs in FP32 when Q_ij Q_kl max|D| < fp32_cut.  The
+  // Schwarz cut fp32_cut / max|D| is rounded down to a power of two (conservative:
+  // fewer FP32 quartets), so that the split, built on the host, is rebuilt only
+  // when max|D| moves past a power of two.
+  double cut = forced_cut >= 0.0 ? forced_cut : 0.0;
+  if (o.fp32_cut > 0.0 && forced_cut < 0.0) {
+    double maxd = 0.0;
+    if (int rc = device_absmax(E, dD, elems, stream, &maxd)) return rc;
+    if (maxd > 0.0 && std::isfinite(maxd)) cut = std::exp2(std::floor(std::log2(o.fp32_cut / maxd)));
+  }
+  if (cut > 0.0)
+    if (int rc = build_split(E, cut)) return rc;
+  lai_jk_report r{};
+  if (int rc = enqueue_jk(E, dD, stream, o, cut, timed, r)) return rc;
   const int64_t nn = (int64_t)elems;
   if (nn > 0) {
     if (batched)
       symmetrize_batched_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, stream>>>(
-          E->d_Jp.as<double>(), E->d_Kp.as<double>(), dJ, dK, E->d_sys_off.as<int64_t>(),
-          E->d_sys_nbf.as<int>(), E->nsys);
+          E->jp(), E->kp(copies * elems), dJ, dK, E->d_sys_off.as<int64_t>(), E->d_sys_nbf.as<int>(), E->nsys, copies);
     else
-      symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, stream>>>(
-          E->d_Jp.as<double>(), E->d_Kp.as<double>(), dJ, dK, nbf);
-    ++launches;
+      symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, stream>>>(E->jp(), E->kp(copies * elems), dJ, dK, nbf,
+                                                                          copies);
+    ++r.kernel_launches;
   }
   LAI_CUDA_TRY(cudaGetLastError());
   if (timed) LAI_CUDA_TRY(cudaEventRecord(E->ev1, stream));
   if (rep) {
-    rep->quartets_fp64 = nq - nq32;
-    rep->quartets_fp32 = nq32;
-    rep->fp32_schwarz_cut = cut;
-    rep->alg_flops = flops;
-    rep->kernel_launches = launches;
-    rep->seconds_device = 0;
+    const double total = rep->seconds_total;
+    *rep = r;
+    rep->seconds_total = total;
   }
   return LAI_OK;
 }
@@ -814,6 +996,7 @@ int create_engine(const lai_basis* basis, std::unique_ptr<lai_basis> merged, con
     return E->blocks[x]->alg_flops * (double)E->blocks[x]->total >
            E->blocks[y]->alg_flops * (double)E->blocks[y]->total;
   });
+  if (int rc = build_launches(E.get())) return rc;
   *out = E.release();
   return LAI_OK;
 }
@@ -1136,13 +1319,14 @@ int lai_engine_autotune(lai_engine* engine, const double* d_D, void* stream, dou
   LAI_CUDA_TRY(dK.alloc(sizeof(double) * elems));
   if (int rc = run_jk(engine, d_D, dJ.as<double>(), dK.as<double>(), s, o, nullptr, false)) return rc;
   engine->release_graph();
+  engine->tuned = true;
   cudaEvent_t e0, e1;
   LAI_CUDA_TRY(cudaEventCreate(&e0));
   LAI_CUDA_TRY(cudaEventCreate(&e1));
   lai::JKArgs args{};
   args.D = d_D;
-  args.J = engine->d_Jp.as<double>();
-  args.K = engine->d_Kp.as<double>();
+  args.J = engine->jp();
+  args.K = engine->kp(elems);
   args.nbf = (int)engine->basis->nbf;
   args.mode = lai::MODE_JK;
   args.prim_eps = engine->prim_eps;
@@ -1200,6 +1384,13 @@ int lai_engine_autotune(lai_engine* engine, const double* d_D, void* stream, dou
         if ((rc = time_launch(q, lai::LaunchTune{ps, ks}, &m))) break;
         if (m < 0.98f * best_ms) { best_ms = m; best = lai::LaunchTune{ps, ks}; }
       }
+    if (!rc && q.total - q.t_begin < (int64_t)engine->num_sms * 64) {
+      float m = 0;
+      lai::LaunchTune t;
+      t.kernel = lai::KERNEL_BLOCK;
+      rc = time_launch(q, t, &m);
+      if (!rc && m < 0.98f * best_ms) { best_ms = m; best = t; }
+    }
     if (rc) break;
     bp->tune = best;
     after += best_ms;

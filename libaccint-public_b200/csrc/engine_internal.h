@@ -169,7 +169,9 @@ struct lai_engine {
   std::vector<std::unique_ptr<lai::host::PairClassHost>> classes;
   std::vector<std::unique_ptr<lai::host::ClassPairBlock>> blocks;
   std::vector<double> Q_all;     // nshell x nshell Schwarz matrix
-  lai::host::DevBuf d_Jp, d_Kp, d_D, d_J, d_K;
+  lai::host::DevBuf d_JKp, d_D, d_J, d_K;
+  double* jp() const { return d_JKp.as<double>(); }
+  double* kp(size_t elems) const { return d_JKp.as<double>() + elems; }  // elems: all of J' (every accumulator)
   lai::host::DevBuf d_scratch;
   size_t scratch_doubles = 0;
   lai::host::DevBuf d_status;
@@ -212,9 +214,23 @@ struct lai_engine {
   int prof_n = 0;
   // streams the independent class-pair launches of one build are spread over
   lai::host::LaneSet lanes;
-  std::recursive_mutex lanes_mutex;   // held while launches are queued on the lanes
+  std::recursive_mutex lanes_mutex;   // held while launches are queued on the lanes, or captured
   cudaStream_t fork_stream = nullptr; // caller's stream while a build is spread over lanes
   std::vector<int> launch_order;      // blocks by descending estimated work
+  // The launches of a plain build (FP64, one shard, untuned), by descending estimated
+  // work: single blocks, and groups of a class's smaller blocks that share a launch
+  // (build_launches).
+  struct LaunchItem {
+    int block = -1;                   // a single block, or
+    bool block_kernel = false;        // a group for the block-per-quartet kernel, or for the split thread-per-quartet one
+    int la = 0, lb = 0, lc = 0, ld = 0;
+    int first = 0, n = 0;             // its entries in d_multi
+    int64_t nwork = 0, Pmax = 0;
+    double work = 0.0;
+  };
+  std::vector<LaunchItem> launches;
+  lai::host::DevBuf d_multi;          // MultiEntry of every group
+  bool tuned = false;                 // lai_engine_autotune has chosen per-block launches
 };
 
 inline lai_engine::~lai_engine() {
@@ -235,6 +251,7 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
                  bool fp32 = false, bool* ran_fp32 = nullptr, lai::LaunchTune tune = lai::LaunchTune{});
 lai::QuartetBlock make_block(const lai_engine* E, const ClassPairBlock& b);
 int ensure_scratch(lai_engine* E, size_t doubles);
+int ensure_accumulators(lai_engine* E, size_t elems);
 
 // Spreads independent launches over the engine's lanes: pick(w) returns the stream of
 // the lane with the least estimated work so far; join() makes the caller's stream wait
@@ -248,7 +265,7 @@ int ensure_scratch(lai_engine* E, size_t doubles);
 // (H2O)64/cc-pVDZ 1505 -> 1390 ms; (H2O)6/cc-pVDZ gradient 82.5 -> 30.5 ms.
 class LaunchLanes {
  public:
-  LaunchLanes(lai_engine* E, cudaStream_t stream, bool spread);
+  LaunchLanes(lai_engine* E, cudaStream_t stream, size_t lanes);
   ~LaunchLanes() { join(); }
   LaunchLanes(const LaunchLanes&) = delete;
   cudaError_t pick(double work, cudaStream_t* s);

@@ -63,7 +63,20 @@ __host__ __device__ constexpr int odd_stride(int n) {
 constexpr int kMaxThreads = 160;  // components of (gg|: 145
 constexpr int kMaxTerms = 12;     // transfer terms of a g component: (2,1,1) -> 3 * 2 * 2
 constexpr int kMaxLab = 2 * kMaxL;
-constexpr int kMaxSmem = 227 * 1024;
+constexpr int kMaxSmem = 226 * 1024;  // of 227 KB, less the static part
+
+// Registers: left alone, ptxas takes 255 for any ket and a block of 32 threads ends up with
+// 8 warps per SM, each waiting on its own arithmetic and shared-memory latency (ncu, (dd|dp):
+// issue active 30 %, stalls `wait` and `short_scoreboard`).  Caps of 96 and 128 registers
+// (65536 / (160 * blocks)) pay for the kets of few components, C6H14/cc-pVTZ without and
+// with them: (fd|ps) 4.9 -> 3.5 ms, (ff|ps) 1.6 -> 0.9, (fs|dp) 4.8 -> 4.0, (fd|pp) 1.75 ->
+// 1.67, but (dd|pp) 2.5 -> 2.8; from 25 components on the spills cost more ((dd|fp) 1.2 ->
+// 1.6 with 128).
+template <int F0, int F1>
+__host__ __device__ constexpr int min_blocks() {
+  constexpr int nf = ncart_range(F0, F1);
+  return nf <= 10 ? 4 : nf <= 16 ? 3 : 1;
+}
 
 __host__ __device__ constexpr int block_binom(int n, int k) {
   int r = 1;
@@ -89,8 +102,6 @@ __host__ __device__ constexpr int chunk_components(int lc, int ld) {
 struct BlockGeom {
   int la, lb, nroots, ne, nab, na, nb;
   int batch;     // primitive quartets per table phase
-  int nsplit;    // blocks that share one quartet's primitive quartets
-  int csplit;    // blocks that share one quartet's ket components
   int chunk;     // consecutive work items a block takes at a time
   int ts;        // one direction's table: (la + lb + 1) * row stride, in values
   int nacc;      // density elements of a quartet: D_ab, D_cd, D_ac, D_ad, D_bc, D_bd
@@ -161,8 +172,9 @@ __device__ __forceinline__ int find_bra_warp(const int64_t* __restrict__ offsets
 }
 
 template <int LC, int LD, int F0, int F1, typename R>
-__global__ void __launch_bounds__(kMaxThreads) eri_block_kernel(QuartetBlock blk, JKArgs args, RysTablesView tab,
-                                                                BlockGeom g) {
+__global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
+    eri_block_kernel(QuartetBlock one, JKArgs args, RysTablesView tab, BlockGeom g, int nsplit1, int csplit1,
+                     const MultiEntry* list_of_blocks, int nblocks, int64_t nwork) {
   constexpr int LCD = LC + LD, W = LCD + 1, WS = odd_stride<R>(W);
   constexpr int NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
   constexpr int CB = chunk_components(LC, LD), NV = CB * ND, NVP = odd_stride(NV);
@@ -256,11 +268,17 @@ __global__ void __launch_bounds__(kMaxThreads) eri_block_kernel(QuartetBlock blk
   }
   __syncthreads();
 
-  const int nbra = blk.bra.npairs, nket = blk.ket.npairs;
-  const int Kab = blk.bra.Ka * blk.bra.Kb, Kcd = blk.ket.Ka * blk.ket.Kb;
-  const int64_t P = (int64_t)Kab * Kcd;
-  const int parts = g.nsplit * g.csplit;
-  const int64_t nwork = (blk.total - blk.t_begin) * parts;
+  // the quartets' block: `one`, or the entry of the list that holds the work item
+  __shared__ MultiEntry entry;
+  if (!list_of_blocks && tid == 0) {
+    entry.blk = one;
+    entry.work0 = 0;
+    entry.nsplit = nsplit1;
+    entry.csplit = csplit1;
+  }
+  __syncthreads();
+  const QuartetBlock& blk = entry.blk;
+  int cur = list_of_blocks ? -1 : 0;
   const int64_t nchunk = (nwork + g.chunk - 1) / g.chunk;
   unsigned int nprim_done = 0;
 
@@ -268,10 +286,27 @@ __global__ void __launch_bounds__(kMaxThreads) eri_block_kernel(QuartetBlock blk
     const int64_t w0 = ch * g.chunk, w1 = min(nwork, w0 + g.chunk);
     int p = -1;
     for (int64_t wi = w0; wi < w1; ++wi) {
-      const int64_t tq = parts == 1 ? wi : wi / parts;
-      const int part = (int)(wi - tq * parts), cpart = part / g.nsplit, split = part - cpart * g.nsplit;
+      if (list_of_blocks) {
+        int e = cur < 0 ? 0 : cur;  // work items only move forward
+        while (e + 1 < nblocks && __ldg(&list_of_blocks[e + 1].work0) <= wi) ++e;
+        if (e != cur) {  // (all are past the last quartet: it ended with a sync)
+          const int* src = reinterpret_cast<const int*>(list_of_blocks + e);
+          for (int i = tid; i < (int)(sizeof(MultiEntry) / sizeof(int)); i += nt)
+            reinterpret_cast<int*>(&entry)[i] = __ldg(src + i);
+          cur = e;
+          p = -1;
+          __syncthreads();
+        }
+      }
+      const int nbra = blk.bra.npairs, nket = blk.ket.npairs;
+      const int Kcd = blk.ket.Ka * blk.ket.Kb;
+      const int Kab = blk.bra.Ka * blk.bra.Kb;
+      const int64_t P = (int64_t)Kab * Kcd;
+      const int nsplit = entry.nsplit, csplit = entry.csplit, parts = nsplit * csplit;
+      const int64_t wl = wi - entry.work0, tq = parts == 1 ? wl : wl / parts;
+      const int part = (int)(wl - tq * parts), cpart = part / nsplit, split = part - cpart * nsplit;
       // this part's ket components [c_begin, c_end), whole chunks
-      const int c_begin = cpart * (NC / CB) / g.csplit * CB, c_end = (cpart + 1) * (NC / CB) / g.csplit * CB;
+      const int c_begin = cpart * (NC / CB) / csplit * CB, c_end = (cpart + 1) * (NC / CB) / csplit * CB;
       const int64_t t = blk.t_begin + tq;
       if (p < 0) p = find_bra_warp(blk.offsets, nbra, t);
       else while (t >= __ldg(blk.offsets + p + 1)) ++p;
@@ -312,14 +347,14 @@ __global__ void __launch_bounds__(kMaxThreads) eri_block_kernel(QuartetBlock blk
       // the cut collected in a list, the list processed `batch` at a time ----
       const double* __restrict__ pbra = blk.bra.primb + (size_t)p * Kab * kBraRec;
       const double* __restrict__ pket = blk.ket.primb + (size_t)q * Kcd * kBraRec;
-      for (int64_t c0 = split; c0 < P; c0 += (int64_t)nt * g.nsplit) {
+      for (int64_t c0 = split; c0 < P; c0 += (int64_t)nt * nsplit) {
         int cnt;
         if (P == 1) {  // (the usual case of the d, f and g shells): no list
           cnt = __ldg(pbra + BR_Q) * __ldg(pket + BR_Q) < args.prim_eps ? 0 : 1;
         } else {
           if (tid == 0) *nlist = 0;
           __syncthreads();
-          const int64_t ci = c0 + (int64_t)tid * g.nsplit;
+          const int64_t ci = c0 + (int64_t)tid * nsplit;
           bool pass = false;
           if (ci < P) {
             const int64_t ib = ci / Kcd, ik = ci - ib * Kcd;
@@ -549,42 +584,79 @@ __global__ void __launch_bounds__(kMaxThreads) eri_block_kernel(QuartetBlock blk
   if (F0 == LC) count_prims(args.prim_count, tid == 0 ? nprim_done : 0u);
 }
 
-// 0 when launched, -3 on a CUDA error.
+// Geometry of a bra and its resident blocks per SM; -3 on a CUDA error.
 template <int LC, int LD, int F0, int F1, typename R>
-int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
-                 int num_sms) {
-  const int la = blk.bra.la, lb = blk.bra.lb;
-  const int threads = (ncart_range(la, la + lb) + 31) / 32 * 32;
+int block_geometry(int la, int lb, int64_t P, BlockGeom* g, int* threads, size_t* smem) {
+  *threads = (ncart_range(la, la + lb) + 31) / 32 * 32;
   const int nroots = (la + lb + LC + LD) / 2 + 1;
-  const int64_t P = (int64_t)blk.bra.Ka * blk.bra.Kb * blk.ket.Ka * blk.ket.Kb;
   // table batch: one thread per (primitive quartet, root, direction); a block of 32 has
   // room for at least one primitive quartet of its class (27 >= 3 nroots)
-  int batch = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(P, 8), threads / (3 * nroots)));
-  BlockGeom g = make_geom<LC, LD, R>(la, lb, threads, batch);
-  while (g.doubles * 8 > kMaxSmem && batch > 1) g = make_geom<LC, LD, R>(la, lb, threads, --batch);
-  const size_t smem = sizeof(double) * (size_t)g.doubles;
+  int batch = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(P, 8), *threads / (3 * nroots)));
+  *g = make_geom<LC, LD, R>(la, lb, *threads, batch);
+  while (g->doubles * 8 > kMaxSmem && batch > 1) *g = make_geom<LC, LD, R>(la, lb, *threads, --batch);
+  *smem = sizeof(double) * (size_t)g->doubles;
   auto kern = eri_block_kernel<LC, LD, F0, F1, R>;
   // resident blocks per SM, per bra and batch (0: not asked yet)
   static std::atomic<int> occ[kMaxL + 1][kMaxL + 1][9];
   int per_sm = occ[la][lb][batch].load(std::memory_order_relaxed);
   if (per_sm == 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, *threads, *smem) != cudaSuccess || per_sm < 1)
       return -3;
     occ[la][lb][batch].store(per_sm, std::memory_order_relaxed);
   }
+  return per_sm;
+}
+
+// Blocks that share a quartet, where a launch has too few quartets (nq) for the `slots`
+// blocks the device holds: first by primitive quartets (at least two table batches each),
+// then by chunks of ket components.
+inline void block_split(int64_t nq, int64_t P, int batch, int nchunks, int64_t slots, int* nsplit, int* csplit) {
+  *nsplit = (int)std::max<int64_t>(1, std::min<int64_t>(P / (2 * batch), slots / nq));
+  *csplit = (int)std::max<int64_t>(1, std::min<int64_t>(nchunks, slots / (nq * *nsplit)));
+}
+
+// 0 when launched, -3 on a CUDA error.
+template <int LC, int LD, int F0, int F1, typename R>
+int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
+                 int num_sms) {
+  const int64_t P = (int64_t)blk.bra.Ka * blk.bra.Kb * blk.ket.Ka * blk.ket.Kb;
+  BlockGeom g;
+  int threads;
+  size_t smem;
+  const int per_sm = block_geometry<LC, LD, F0, F1, R>(blk.bra.la, blk.bra.lb, P, &g, &threads, &smem);
+  if (per_sm < 0) return per_sm;
   const int64_t nq = blk.total - blk.t_begin, slots = (int64_t)num_sms * per_sm;
-  // too few quartets for the device: blocks share a quartet's primitive quartets, at
-  // least two table batches each, and then its chunks of ket components
-  g.nsplit = (int)std::max<int64_t>(1, std::min<int64_t>(P / (2 * batch), slots / nq));
-  g.csplit = (int)std::max<int64_t>(1, std::min<int64_t>(ncart(LC) / chunk_components(LC, LD),
-                                                         slots / (nq * g.nsplit)));
-  const int64_t nwork = nq * g.nsplit * g.csplit;
+  int nsplit, csplit;
+  block_split(nq, P, g.batch, ncart(LC) / chunk_components(LC, LD), slots, &nsplit, &csplit);
+  const int64_t nwork = nq * nsplit * csplit;
   // consecutive quartets per block (one search for the bra pair, its data cached), at
   // least eight turns per block for balance
   g.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, nwork / (slots * 8)));
   const int64_t want = (nwork + g.chunk - 1) / g.chunk;
-  kern<<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(blk, args, tab, g);
+  eri_block_kernel<LC, LD, F0, F1, R><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
+      blk, args, tab, g, nsplit, csplit, nullptr, 0, nwork);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// The n blocks of a list (device memory; one bra (la, lb), Pmax the most primitive quartets
+// of an entry) as one launch of nwork work items.
+template <int LC, int LD, int F0, int F1>
+int launch_range_list(int la, int lb, int64_t Pmax, const MultiEntry* list, int n, int64_t nwork, const JKArgs& args,
+                      const RysTablesView& tab, cudaStream_t stream, int num_sms) {
+  BlockGeom g;
+  int threads;
+  size_t smem;
+  const int per_sm = block_geometry<LC, LD, F0, F1, double>(la, lb, Pmax, &g, &threads, &smem);
+  if (per_sm < 0) return per_sm;
+  const int64_t slots = (int64_t)num_sms * per_sm;
+  g.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, nwork / (slots * 8)));
+  // few work items: four to a block, which then sets up its class tables once for them
+  // (the launches of other classes fill the device meanwhile)
+  const int64_t want = std::max<int64_t>(std::min<int64_t>(num_sms, nwork), (nwork + 4 * g.chunk - 1) / (4 * g.chunk));
+  eri_block_kernel<LC, LD, F0, F1, double><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
+      QuartetBlock{}, args, tab, g, 1, 1, list, n, nwork);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

@@ -7,10 +7,14 @@ namespace block_detail {
 
 template int launch_range<2, 1, 2, 3, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
+template int launch_range_list<2, 1, 2, 3>(int, int, int64_t, const MultiEntry*, int, int64_t,
+                                          const JKArgs&, const RysTablesView&, cudaStream_t, int);
 template int launch_range<2, 1, 2, 3, float>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
 template int launch_range<3, 1, 3, 4, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
+template int launch_range_list<3, 1, 3, 4>(int, int, int64_t, const MultiEntry*, int, int64_t,
+                                          const JKArgs&, const RysTablesView&, cudaStream_t, int);
 template int launch_range<3, 1, 3, 4, float>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
 

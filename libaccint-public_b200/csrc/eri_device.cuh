@@ -96,6 +96,11 @@ struct JKArgs {
   double prim_eps;       // skip primitive quartets with q_ab * q_cd < prim_eps (0 = none)
   double prim_rel32;     // FP32 kernels: also skip q_ab * q_cd < prim_rel32 * Q_ij * Q_kl
   unsigned long long* prim_count;  // optional: += primitive quartets executed by the launch
+  // J and K each hold copy_mask + 1 (a power of two) accumulators, copy_stride doubles
+  // apart, that the caller sums; a block adds to accumulator blockIdx.x & copy_mask.  (One
+  // long sum carries more rounding error than several short ones.)
+  int copy_mask;
+  int64_t copy_stride;
   // batched engines (many independent systems): D, J and K hold one nbf_s x nbf_s
   // block per system, block s at element offset sys_off[s]; function indices are
   // local to the system.  nullptr for a single system.
@@ -111,7 +116,8 @@ struct SysMats {
   int nbf;
 };
 __device__ __forceinline__ SysMats sys_mats(const JKArgs& args, const QuartetBlock& blk, int p) {
-  SysMats m{args.D, args.J, args.K, args.nbf};
+  const int64_t copy = (int64_t)(blockIdx.x & args.copy_mask) * args.copy_stride;
+  SysMats m{args.D, args.J + copy, args.K + copy, args.nbf};
   if (blk.bra.sys) {
     const int s = __ldg(blk.bra.sys + p);
     const int64_t o = __ldg(args.sys_off + s);

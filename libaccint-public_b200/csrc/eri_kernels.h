@@ -20,6 +20,21 @@ struct LaunchTune {
                    // KERNEL_TILED, KERNEL_SLICED or KERNEL_BLOCK
 };
 enum { KERNEL_DEFAULT = 0, KERNEL_TILED = 2, KERNEL_SLICED = 3, KERNEL_BLOCK = 4 };
+// One of several blocks of a class that share a launch: work items [work0, next entry's
+// work0) are its chunks of 32 / ps quartets, nsplit parts by ket primitive each
+// (thread-per-quartet kernels), or its quartets times nsplit * csplit parts
+// (block-per-quartet kernel).
+struct MultiEntry {
+  QuartetBlock blk;
+  int64_t work0;
+  int ps;
+  int nsplit, csplit;
+  int pad;
+};
+// A launch with fewer quartets per SM than this splits them over lanes.
+constexpr int kSplitQuartetsPerSm = 1024;
+int launch_small_list(int la, int lb, int lc, int ld, const MultiEntry* list, int n, int64_t nwork,
+                      const JKArgs& args, const RysTablesView& tab, cudaStream_t stream, int num_sms);
 int launch_small(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,
                  cudaStream_t stream, bool fp32, int num_sms, LaunchTune tune = LaunchTune{});
 bool small_class_supported(int la, int lb, int lc, int ld);
@@ -43,7 +58,12 @@ int launch_tiled(const QuartetBlock& blk, const JKArgs& args, const RysTablesVie
 // fp32 asks for the FP32 variant (block_fp32_class).
 int launch_blockq(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
                   int num_sms, bool fp32);
+int launch_blockq_list(int la, int lb, int lc, int ld, int64_t Pmax, const MultiEntry* list, int n, int64_t nwork,
+                       const JKArgs& args, const RysTablesView& tab, cudaStream_t stream, int num_sms);
+int block_ket_chunks(int lc, int ld);  // digestion chunks of a ket, the most parts of csplit
 bool block_fp32_class(int la, int lb, int lc, int ld);
+// whether a J/K launch of a thread-per-quartet class goes to the block-per-quartet kernel
+bool block_for_few(const QuartetBlock& blk, int num_sms);
 
 // Warp-per-quartet generic kernel (eri_generic.cu), any class with l <= 4.
 int launch_generic(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,

@@ -1,4 +1,4 @@
-// Explicit instantiations of the small-class kernels (part 5 of 6; split so
+// Explicit instantiations of the small-class kernels (part 5 of 9; split so
 // nvcc compiles the classes in parallel).
 #include "eri_small_impl.cuh"
 
@@ -7,10 +7,16 @@ namespace small_detail {
 
 template int launch_one<1, 1, 1, 0>(const QuartetBlock&, const JKArgs&, const RysTablesView&,
                                    cudaStream_t, bool, int, LaunchTune);
+template int launch_list<1, 1, 1, 0>(const MultiEntry*, int, int64_t, const JKArgs&, const RysTablesView&,
+                                    cudaStream_t, int);
 template int launch_one<3, 0, 0, 0>(const QuartetBlock&, const JKArgs&, const RysTablesView&,
                                    cudaStream_t, bool, int, LaunchTune);
+template int launch_list<3, 0, 0, 0>(const MultiEntry*, int, int64_t, const JKArgs&, const RysTablesView&,
+                                    cudaStream_t, int);
 template int launch_one<2, 1, 1, 0>(const QuartetBlock&, const JKArgs&, const RysTablesView&,
                                    cudaStream_t, bool, int, LaunchTune);
+template int launch_list<2, 1, 1, 0>(const MultiEntry*, int, int64_t, const JKArgs&, const RysTablesView&,
+                                    cudaStream_t, int);
 
 }  // namespace small_detail
 }  // namespace lai

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "eri_device.cuh"
@@ -103,10 +104,12 @@ template <int LA, int LB, int LC, int LD, typename R, bool SPLIT>
 __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKArgs& args,
                                               const RysTablesView& tab,
                                               const R* __restrict__ stab, int64_t t, int p,
-                                              bool active, bool uniform_bra, int ps, int sub) {
+                                              bool active, bool uniform_bra, int ps, int sub, int ks, int kpart) {
   // ps lanes (a power of two, aligned) share this quartet: lane `sub` of the group
   // runs bra primitive pairs sub, sub+ps, ...; the group then sums its partial
-  // (e0|f0) blocks and lane 0 of the group alone transfers and digests.
+  // (e0|f0) blocks and lane 0 of the group alone transfers and digests.  ks work items
+  // share it too: this one runs ket primitive pairs kpart, kpart + ks, ... and digests
+  // its part (everything after the primitive sum is linear in it).
   constexpr int LAB = LA + LB, LCD = LC + LD;
   constexpr int NR = (LAB + LCD) / 2 + 1;
   constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
@@ -156,6 +159,7 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
   unsigned int nprim_done = 0;
   // unsplit: compile-time stride 1 keeps the bra loop warp-uniform
   const int ib0 = SPLIT ? sub : 0, ibs = SPLIT ? ps : 1;
+  const int ik0 = SPLIT ? kpart : 0, iks = SPLIT ? ks : 1;
   // One primitive quartet: bra primitive pair (zeta, hz, PA, cab), ket
   // primitive pair `cur`; accumulates into G.  The FP32 kernels read an FP32 copy
   // of the pair tables (half the bytes and registers, no conversions).
@@ -376,7 +380,8 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
   // primitives (s pairs against p/d pairs) and goes inside, with its next primitive
   // pair loaded one iteration ahead.
   // this lane's ket pair in the ket tiles: primitive ik at pkt + ik * kKetPrimStride
-  const R* __restrict__ pkt = ket_tile_ptr(ket_tiles<R>(blk.ket), q, Kcd);
+  const R* __restrict__ pkt = ket_tile_ptr(ket_tiles<R>(blk.ket), q, Kcd) + (size_t)ik0 * kKetPrimStride;
+  const size_t kstep = (size_t)iks * kKetPrimStride;
   // FP32 quartets (fp32_prim_rel > 0): primitive quartets below that fraction of the
   // quartet's own Schwarz bound are skipped as well
   const R peps_r = R((F32 && args.prim_rel32 > 0.0)
@@ -386,10 +391,12 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
     const R qab_max = ib0 < Kab ? __ldg(bprim + (size_t)ib0 * nbra + p + PF_Q * sb) : R(0);
     KetPrimT<R> nxt;
     load_ket_rec(pkt, nxt);
-    for (int ik = 0; ik < Kcd; ++ik) {
+    const R* __restrict__ pk = pkt;
+    for (int ik = ik0; ik < Kcd; ik += iks) {
       const KetPrimT<R> cur = nxt;
       if (qab_max * cur.q < peps_r || ib0 >= Kab) break;
-      if (ik + 1 < Kcd) load_ket_rec(pkt + (size_t)(ik + 1) * kKetPrimStride, nxt);
+      pk += kstep;
+      if (ik + iks < Kcd) load_ket_rec(pk, nxt);
       BraVals bv{};
       for (int ib = ib0; ib < Kab; ib += ibs) {
         R qab;
@@ -413,12 +420,14 @@ __device__ __forceinline__ void small_quartet(const QuartetBlock& blk, const JKA
       load_bra(ib, qab, bv);
       if (qab * qket_max < peps_r) break;
       KetPrimT<R> nxt = k0;
-      for (int ik = 0; ik < Kcd; ++ik) {
-        if constexpr (!kAhead) load_ket_rec(pkt + (size_t)ik * kKetPrimStride, nxt);
+      const R* __restrict__ pk = pkt;
+      for (int ik = ik0; ik < Kcd; ik += iks) {
+        if constexpr (!kAhead) load_ket_rec(pk, nxt);
         const KetPrimT<R> cur = nxt;
         if (qab * cur.q < peps_r) break;
+        pk += kstep;
         if constexpr (kAhead)
-          if (ik + 1 < Kcd) load_ket_rec(pkt + (size_t)(ik + 1) * kKetPrimStride, nxt);
+          if (ik + iks < Kcd) load_ket_rec(pk, nxt);
         ++nprim_done;
         prim(bv, cur);
       }
@@ -711,47 +720,91 @@ __host__ __device__ constexpr int small_min_blocks() {
                         : (L <= 1 ? 4 : L == 2 ? 2 : 0);
 }
 
+// SPLIT = false: one block of quartets, a thread per quartet.  SPLIT = true: the n blocks
+// of `list` (or `blk` alone), each with its own number of lanes per quartet, as one launch:
+// the class's small launches (an engine has one per pair of primitive counts) would each
+// stage the lookup table and fill a few warps.
 template <int LA, int LB, int LC, int LD, typename R, bool SPLIT>
 __global__ void __launch_bounds__(256, (small_min_blocks<LA, LB, LC, LD, R>()))
-    eri_small_kernel(QuartetBlock blk, JKArgs args, RysTablesView tab, int kSuper, int ps) {
+    eri_small_kernel(QuartetBlock blk, JKArgs args, RysTablesView tab, int kSuper, int ps, const MultiEntry* list,
+                     int n, int64_t nwork) {
   constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* stab = reinterpret_cast<R*>(smem_raw);
   if constexpr (sizeof(R) == 4) stage_table_f32<NR>(reinterpret_cast<float*>(smem_raw), tab);
   else if constexpr (small_boys<LA, LB, LC, LD, R>()) stage_boys_rows<LA + LB + LC + LD>(stab, tab);
   else stage_table<NR, R>(stab, tab);
-  __syncthreads();
   const int lane = threadIdx.x & 31;
-  if (!SPLIT) ps = 1;
-  const int qpw = 32 / ps;  // quartets per warp chunk
-  const int slot = lane / ps, sub = lane & (ps - 1);
-  const int64_t nq = blk.total - blk.t_begin;
-  const int64_t nchunks = (nq + qpw - 1) / qpw;
   const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int nbra = blk.bra.npairs;
-  // grid-stride over super-chunks of kSuper chunks (load balance), one bra search
-  // per super-chunk, then the bra index only moves forward
-  const int64_t nsuper = (nchunks + kSuper - 1) / kSuper;
-  for (int64_t sc = wid; sc < nsuper; sc += nw) {
-    const int64_t c1 = min(nchunks, (sc + 1) * kSuper);
-    int pw = -1;  // bra pair of the current chunk's first quartet
-    for (int64_t c = sc * kSuper; c < c1; ++c) {
-      const int64_t t0 = blk.t_begin + c * qpw;
-      const int64_t t = t0 + slot;
-      const bool active = t < blk.total;
-      const int64_t te = active ? t : blk.total - 1;
-      if (pw < 0) {
-        if (lane == 0) pw = find_bra(blk.offsets, nbra, t0);
-        pw = __shfl_sync(0xffffffffu, pw, 0);
-      } else {
-        while (t0 >= __ldg(blk.offsets + pw + 1)) ++pw;
+  if constexpr (SPLIT) {
+    __shared__ MultiEntry entries[8];  // each warp's current block
+    MultiEntry& en = entries[threadIdx.x >> 5];
+    if (!list && lane == 0) {
+      en.blk = blk;
+      en.ps = ps;
+      en.nsplit = 1;
+      en.work0 = 0;
+    }
+    __syncthreads();
+    int cur = list ? -1 : 0;
+    for (int64_t c = wid; c < nwork; c += nw) {
+      if (list) {
+        int e = cur < 0 ? 0 : cur;  // chunks only move forward
+        while (e + 1 < n && __ldg(&list[e + 1].work0) <= c) ++e;
+        if (e != cur) {
+          __syncwarp();
+          const int* src = reinterpret_cast<const int*>(list + e);
+          for (int i = lane; i < (int)(sizeof(MultiEntry) / sizeof(int)); i += 32)
+            reinterpret_cast<int*>(&en)[i] = __ldg(src + i);
+          cur = e;
+          __syncwarp();
+        }
       }
+      const int lps = en.ps, qpw = 32 / lps;  // lanes per quartet, quartets per chunk
+      const int slot = lane / lps, sub = lane & (lps - 1);
+      const int64_t cl = c - en.work0, ck = en.nsplit == 1 ? cl : cl / en.nsplit;
+      const int kpart = (int)(cl - ck * en.nsplit);
+      const int64_t t0 = en.blk.t_begin + ck * qpw;
+      const bool active = t0 + slot < en.blk.total;
+      const int64_t te = active ? t0 + slot : en.blk.total - 1;
+      int pw = 0;
+      if (lane == 0) pw = find_bra(en.blk.offsets, en.blk.bra.npairs, t0);
+      pw = __shfl_sync(0xffffffffu, pw, 0);
       int p = pw;
-      while (te >= __ldg(blk.offsets + p + 1)) ++p;
+      while (te >= __ldg(en.blk.offsets + p + 1)) ++p;
       const bool uniform = __all_sync(0xffffffffu, p == pw);
-      small_quartet<LA, LB, LC, LD, R, SPLIT>(blk, args, tab, stab, te, p, active, uniform,
-                                              SPLIT ? ps : 1, SPLIT ? sub : 0);
+      small_quartet<LA, LB, LC, LD, R, true>(en.blk, args, tab, stab, te, p, active, uniform, lps, sub,
+                                               en.nsplit, kpart);
+    }
+  } else {
+    __syncthreads();
+    const int64_t nq = blk.total - blk.t_begin;
+    const int64_t nchunks = (nq + 31) / 32;
+    const int nbra = blk.bra.npairs;
+    // grid-stride over super-chunks of kSuper chunks (load balance), one bra search
+    // per super-chunk, then the bra index only moves forward
+    const int64_t nsuper = (nchunks + kSuper - 1) / kSuper;
+    for (int64_t sc = wid; sc < nsuper; sc += nw) {
+      const int64_t c1 = min(nchunks, (sc + 1) * kSuper);
+      int pw = -1;  // bra pair of the current chunk's first quartet
+      for (int64_t c = sc * kSuper; c < c1; ++c) {
+        const int64_t t0 = blk.t_begin + c * 32;
+        const int64_t t = t0 + lane;
+        const bool active = t < blk.total;
+        const int64_t te = active ? t : blk.total - 1;
+        if (pw < 0) {
+          if (lane == 0) pw = find_bra(blk.offsets, nbra, t0);
+          pw = __shfl_sync(0xffffffffu, pw, 0);
+        } else {
+          while (t0 >= __ldg(blk.offsets + pw + 1)) ++pw;
+        }
+        int p = pw;
+        while (te >= __ldg(blk.offsets + p + 1)) ++p;
+        const bool uniform = __all_sync(0xffffffffu, p == pw);
+        small_quartet<LA, LB, LC, LD, R, false>(blk, args, tab, stab, te, p, active, uniform, 1, 0, 1,
+                                                0);
+      }
     }
   }
 }
@@ -760,38 +813,47 @@ __global__ void __launch_bounds__(256, (small_min_blocks<LA, LB, LC, LD, R>()))
 
 namespace small_detail {
 
+// The kernel of a variant (0: FP64, 1: FP64 split, 2: FP32, 3: FP32 split) and its
+// resident blocks per SM; -3 on a CUDA error.  Separate instantiations keep the unsplit
+// kernel's register allocation independent of the split one.
+using SmallKernel = void (*)(QuartetBlock, JKArgs, RysTablesView, int, int, const MultiEntry*, int, int64_t);
+constexpr int kSmallThreads = 256;
+template <int LA, int LB, int LC, int LD>
+int small_variant(int v, SmallKernel* kern, size_t* smem) {
+  const SmallKernel kerns[4] = {
+      eri_small_kernel<LA, LB, LC, LD, double, false>, eri_small_kernel<LA, LB, LC, LD, double, true>,
+      eri_small_kernel<LA, LB, LC, LD, float, false>, eri_small_kernel<LA, LB, LC, LD, float, true>};
+  *kern = kerns[v];
+  *smem = v >= 2 ? small_table_bytes<LA, LB, LC, LD, float>() : small_table_bytes<LA, LB, LC, LD, double>();
+  static std::atomic<int> per_sm[4];
+  int n = per_sm[v].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaFuncSetAttribute(kerns[v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kerns[v], kSmallThreads, *smem) != cudaSuccess)
+      return -3;
+    n = std::max(n, 1);
+    per_sm[v].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 template <int LA, int LB, int LC, int LD>
 int launch_one(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,
                cudaStream_t stream, bool fp32, int num_sms, LaunchTune tune) {
-  const int threads = 256;
-  const size_t smem = fp32 ? small_table_bytes<LA, LB, LC, LD, float>() : small_table_bytes<LA, LB, LC, LD, double>();
   const int64_t nq = blk.total - blk.t_begin;
   if (nq <= 0) return 1;
   // lanes per quartet: split the bra primitive loop when the launch has too few
   // quartets to fill the device (primitive-heavy classes such as (s9 s9|s9 s9))
   const int Kab = blk.bra.Ka * blk.bra.Kb;
   int ps = 1;
-  while (ps < 32 && ps < Kab && nq * ps < (int64_t)num_sms * 1024) ps <<= 1;
+  while (ps < 32 && ps < Kab && nq * ps < (int64_t)num_sms * kSplitQuartetsPerSm) ps <<= 1;
   if (tune.ps > 0) ps = tune.ps;
   const int64_t nchunks = (nq + 32 / ps - 1) / (32 / ps);
-  // separate instantiations keep the unsplit kernel's register allocation
-  // independent of the split one
-  const int v = (fp32 ? 2 : 0) + (ps > 1 ? 1 : 0);
-  void (*const kerns[4])(QuartetBlock, JKArgs, RysTablesView, int, int) = {
-      eri_small_kernel<LA, LB, LC, LD, double, false>, eri_small_kernel<LA, LB, LC, LD, double, true>,
-      eri_small_kernel<LA, LB, LC, LD, float, false>, eri_small_kernel<LA, LB, LC, LD, float, true>};
-  auto kern = kerns[v];
-  static bool attr[4] = {false, false, false, false};
-  static int per_sm_cache[4] = {0, 0, 0, 0};
-  if (!attr[v]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return -3;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_cache[v], kern, threads, smem) != cudaSuccess)
-      return -3;
-    attr[v] = true;
-  }
-  const int per_sm = per_sm_cache[v] > 0 ? per_sm_cache[v] : 1;
-  const int64_t want = (nchunks + (threads / 32) - 1) / (threads / 32);
+  SmallKernel kern;
+  size_t smem;
+  const int per_sm = small_variant<LA, LB, LC, LD>((fp32 ? 2 : 0) + (ps > 1 ? 1 : 0), &kern, &smem);
+  if (per_sm < 0) return per_sm;
+  const int64_t want = (nchunks + (kSmallThreads / 32) - 1) / (kSmallThreads / 32);
   const int64_t cap = (int64_t)num_sms * per_sm;
   const int grid = (int)(want < cap ? want : cap);
   // chunks per super-chunk (consecutive chunks a warp takes, one bra search per
@@ -801,11 +863,25 @@ int launch_one(const QuartetBlock& blk, const JKArgs& args, const RysTablesView&
   // super-chunks per warp for load balance, so small launches stay at 1.
   int ksuper = tune.ksuper;
   if (ksuper <= 0) {
-    const int64_t warps = (int64_t)grid * (threads / 32);
+    const int64_t warps = (int64_t)grid * (kSmallThreads / 32);
     const int64_t kmax = (int64_t)Kab * blk.ket.Ka * blk.ket.Kb <= 9 ? 16 : 4;
     ksuper = (int)std::max<int64_t>(1, std::min<int64_t>(kmax, nchunks / (warps * 8)));
   }
-  kern<<<grid, threads, smem, stream>>>(blk, args, tab, ksuper, ps);
+  kern<<<grid, kSmallThreads, smem, stream>>>(blk, args, tab, ksuper, ps, nullptr, 0, nchunks);
+  return cudaGetLastError() == cudaSuccess ? 1 : -3;
+}
+
+template <int LA, int LB, int LC, int LD>
+int launch_list(const MultiEntry* list, int n, int64_t nwork, const JKArgs& args, const RysTablesView& tab,
+                cudaStream_t stream, int num_sms) {
+  if (nwork <= 0) return 1;
+  SmallKernel kern;
+  size_t smem;
+  const int per_sm = small_variant<LA, LB, LC, LD>(1, &kern, &smem);
+  if (per_sm < 0) return per_sm;
+  const int64_t want = (nwork + (kSmallThreads / 32) - 1) / (kSmallThreads / 32);
+  kern<<<(unsigned)std::min<int64_t>(want, (int64_t)num_sms * per_sm), kSmallThreads, smem, stream>>>(
+      QuartetBlock{}, args, tab, 1, 1, list, n, nwork);
   return cudaGetLastError() == cudaSuccess ? 1 : -3;
 }
 

@@ -71,7 +71,7 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
   double* const acc = static_cast<double*>(copies.p);
   LAI_CUDA_TRY(cudaMemsetAsync(acc, 0, bytes, stream_of_call));
   const int nbf = (int)engine->basis->nbf;
-  LaunchLanes lanes(engine, stream_of_call, true);
+  LaunchLanes lanes(engine, stream_of_call, kLanes);
   for (const int b : engine->launch_order) {
     const auto& bp = engine->blocks[b];
     const lai::QuartetBlock q = make_block(engine, *bp);

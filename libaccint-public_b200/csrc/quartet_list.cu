@@ -319,26 +319,21 @@ int lai_jk_accumulate_quartets_device(lai_engine* engine, const int32_t* quartet
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   StreamSwap sw(engine, s);
   if (canonical_symmetry) {
-    const size_t bytes = sizeof(double) * (size_t)nbf * nbf;
-    if (engine->d_Jp.bytes < bytes) {
-      engine->release_graph();
-      LAI_CUDA_TRY(engine->d_Jp.alloc(bytes));
-      LAI_CUDA_TRY(engine->d_Kp.alloc(bytes));
-    }
-    LAI_CUDA_TRY(cudaMemsetAsync(engine->d_Jp.p, 0, bytes, s));
-    LAI_CUDA_TRY(cudaMemsetAsync(engine->d_Kp.p, 0, bytes, s));
+    const size_t elems = (size_t)nbf * nbf;
+    if (int rc = ensure_accumulators(engine, elems)) return rc;
+    LAI_CUDA_TRY(cudaMemsetAsync(engine->d_JKp.p, 0, 2 * sizeof(double) * elems, s));
     lai::JKArgs args{};
     args.mode = lai::MODE_JK;
     args.D = d_D;
-    args.J = engine->d_Jp.as<double>();
-    args.K = engine->d_Kp.as<double>();
+    args.J = engine->jp();
+    args.K = engine->kp(elems);
     args.nbf = nbf;
     args.prim_eps = 0.0;
     for (auto& gp : groups)
       if (int rc = launch_block(engine, group_block(*gp), args)) return rc;
     const int64_t nn = (int64_t)nbf * nbf;
     add_symmetrized_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(
-        engine->d_Jp.as<double>(), engine->d_Kp.as<double>(), d_J, d_K, nbf);
+        engine->jp(), engine->kp(elems), d_J, d_K, nbf);
     LAI_CUDA_TRY(cudaGetLastError());
     // the ad-hoc pair tables are freed on return: wait for the kernels
     LAI_CUDA_TRY(cudaStreamSynchronize(s));

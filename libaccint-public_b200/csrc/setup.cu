@@ -340,7 +340,7 @@ int setup_pairs(lai_engine* E) {
     build_tables_kernel<<<blocks_for(nelem), 256, 0, s>>>(d_meta.as<ClassTables>(), nc, nelem, dp, nullptr, nullptr,
                                                           nullptr, ds, de, dcf);
     LAI_CUDA_TRY(cudaGetLastError());
-    LaunchLanes lanes(E, s, true);
+    LaunchLanes lanes(E, s, kLanes);
     for (int c = nc - 1; c >= 0; --c) {
       if (v[c].npairs == 0) continue;
       lai::QuartetBlock blk{};
