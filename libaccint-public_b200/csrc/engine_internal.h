@@ -87,6 +87,7 @@ struct LaneSet {
   cudaEvent_t t0 = nullptr, t1 = nullptr;  // timed builds
 };
 constexpr int kLanes = 8;
+constexpr int kPlanLanes = 32;  // branches of a captured build (a graph's are not bound to hardware queues)
 constexpr size_t kPooledLaneSets = 4;
 int acquire_lanes(LaneSet& out);
 void release_lanes(LaneSet& set);
@@ -201,9 +202,28 @@ struct lai_engine {
   cudaGraphExec_t graph_exec = nullptr;
   GraphKey graph_key{};
   lai_jk_report graph_report{};
+  // The launches of a build as a graph over d_plan_D, for one set of options (build_plan).
+  struct Plan {
+    cudaGraphExec_t exec = nullptr;
+    bool seen = false;
+    double cut = 0.0, fp32_prim_rel = 0.0;
+    int shard_index = 0, shard_count = 1;
+    lai_jk_report report{};
+    bool matches(const lai_jk_opts& o, double c) const {
+      return seen && cut == c && shard_index == o.shard_index && shard_count == o.shard_count &&
+             fp32_prim_rel == o.fp32_prim_rel;
+    }
+    void release() {
+      if (exec) cudaGraphExecDestroy(exec);
+      exec = nullptr;
+      seen = false;
+    }
+  } plan;
+  lai::host::DevBuf d_plan_D;
   void release_graph() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     graph_exec = nullptr;
+    plan.release();
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // per-launch profile of the last build with opts.profile

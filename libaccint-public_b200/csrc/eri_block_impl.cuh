@@ -652,9 +652,7 @@ int launch_range_list(int la, int lb, int64_t Pmax, const MultiEntry* list, int 
   if (per_sm < 0) return per_sm;
   const int64_t slots = (int64_t)num_sms * per_sm;
   g.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, nwork / (slots * 8)));
-  // few work items: four to a block, which then sets up its class tables once for them
-  // (the launches of other classes fill the device meanwhile)
-  const int64_t want = std::max<int64_t>(std::min<int64_t>(num_sms, nwork), (nwork + 4 * g.chunk - 1) / (4 * g.chunk));
+  const int64_t want = (nwork + g.chunk - 1) / g.chunk;
   eri_block_kernel<LC, LD, F0, F1, double><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
       QuartetBlock{}, args, tab, g, 1, 1, list, n, nwork);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

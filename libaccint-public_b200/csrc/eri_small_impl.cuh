@@ -842,17 +842,34 @@ int launch_one(const QuartetBlock& blk, const JKArgs& args, const RysTablesView&
                cudaStream_t stream, bool fp32, int num_sms, LaunchTune tune) {
   const int64_t nq = blk.total - blk.t_begin;
   if (nq <= 0) return 1;
-  // lanes per quartet: split the bra primitive loop when the launch has too few
-  // quartets to fill the device (primitive-heavy classes such as (s9 s9|s9 s9))
+  // lanes per quartet: split the bra primitive loop where the launch does not fill the
+  // device's lanes often enough.  Model: waves of resident lanes times a lane's share of
+  // the quartet, 0.4 of the primitive quartets (what passes the cut) and 12 primitive
+  // quartets' worth of transfer and digestion.  On (H2O)8/STO-3G it picks what the
+  // autotuner measured fastest, 1 - 4 lanes; a fixed count of lanes per SM gave (pp|ss)
+  // and (pp|ps), with 512 and 256 resident lanes, 16: 56 and 62 us against 37 and 35.
   const int Kab = blk.bra.Ka * blk.bra.Kb;
-  int ps = 1;
-  while (ps < 32 && ps < Kab && nq * ps < (int64_t)num_sms * kSplitQuartetsPerSm) ps <<= 1;
-  if (tune.ps > 0) ps = tune.ps;
-  const int64_t nchunks = (nq + 32 / ps - 1) / (32 / ps);
   SmallKernel kern;
   size_t smem;
-  const int per_sm = small_variant<LA, LB, LC, LD>((fp32 ? 2 : 0) + (ps > 1 ? 1 : 0), &kern, &smem);
+  int per_sm = small_variant<LA, LB, LC, LD>(fp32 ? 3 : 1, &kern, &smem);
   if (per_sm < 0) return per_sm;
+  const int64_t lanes = (int64_t)num_sms * per_sm * kSmallThreads;
+  const double P = (double)Kab * blk.ket.Ka * blk.ket.Kb;
+  int ps = 1;
+  double best = 1e300;
+  for (int n = 1; n <= 32 && n < 2 * Kab && (n == 1 || nq * n <= 4 * lanes); n <<= 1) {
+    const double cost = (double)((nq * n + lanes - 1) / lanes) * (0.4 * P / n + 12.0);
+    if (cost < best) {
+      best = cost;
+      ps = n;
+    }
+  }
+  if (tune.ps > 0) ps = tune.ps;
+  const int64_t nchunks = (nq + 32 / ps - 1) / (32 / ps);
+  if (ps == 1) {
+    per_sm = small_variant<LA, LB, LC, LD>(fp32 ? 2 : 0, &kern, &smem);
+    if (per_sm < 0) return per_sm;
+  }
   const int64_t want = (nchunks + (kSmallThreads / 32) - 1) / (kSmallThreads / 32);
   const int64_t cap = (int64_t)num_sms * per_sm;
   const int grid = (int)(want < cap ? want : cap);

@@ -1,0 +1,67 @@
+"""Repeated builds (captured at the second one with the same options) against the first,
+with options and densities that change in between, on several streams, and inside a
+caller's own capture."""
+import importlib
+
+import numpy as np
+import pytest
+
+lai = importlib.import_module("libaccint-public_b200")
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-13  # the launches' atomics add in another order
+
+
+def test_repeated_builds():
+    import torch
+    w = lai.workloads.make("h2o2_631g")
+    n = w.basis.nbf
+    rng = np.random.default_rng(3)
+    dens = [w.D, lai.molecules.random_density(n, 7, rng)]
+    want = []
+    for D in dens:
+        e = lai.Engine(w.basis)
+        want.append([x.copy() for x in e.jk(D)[:2]] + [x.copy() for x in e.jk(D, fp32_cut=1e-6)[:2]])
+    eng = lai.Engine(w.basis)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def build(k, s, cut):
+        with torch.cuda.stream(s):
+            d = torch.from_numpy(dens[k]).cuda()
+            J, K = torch.empty_like(d), torch.empty_like(d)
+            rep = eng.jk_device(d.data_ptr(), J.data_ptr(), K.data_ptr(), stream=s.cuda_stream, fp32_cut=cut)
+            return J.cpu().numpy(), K.cpu().numpy(), rep
+
+    counts = set()
+    for step, (k, s, cut) in enumerate([(0, 0, 0.0), (0, 0, 0.0), (1, 0, 0.0), (1, 1, 0.0), (0, 1, 1e-6),
+                                        (0, 0, 1e-6), (1, 0, 1e-6), (0, 0, 0.0), (1, 1, 0.0), (1, 0, 0.0)]):
+        J, K, rep = build(k, streams[s], cut)
+        Jw, Kw = want[k][2:] if cut else want[k][:2]
+        bar = REL if not cut else 1e-9  # another lane split regroups the FP32 sums
+        assert np.max(np.abs(J - Jw)) < bar * np.max(np.abs(Jw)), step
+        assert np.max(np.abs(K - Kw)) < bar * np.max(np.abs(Jw)), step
+        counts.add(rep.quartets_fp64 + rep.quartets_fp32)
+    assert len(counts) == 1
+
+
+def test_build_inside_a_callers_capture():
+    import torch
+    w = lai.workloads.make("h2o2_631g")
+    eng = lai.Engine(w.basis)
+    Jw, Kw, _ = eng.jk(w.D)
+    eng.jk(w.D)
+    d = torch.from_numpy(w.D).cuda()
+    J, K = torch.empty_like(d), torch.empty_like(d)
+    g = torch.cuda.CUDAGraph()
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+        eng.jk_device(d.data_ptr(), J.data_ptr(), K.data_ptr(), stream=s.cuda_stream)
+    for _ in range(2):
+        J.zero_()
+        K.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.max(np.abs(J.cpu().numpy() - Jw)) < REL * np.max(np.abs(Jw))
+        assert np.max(np.abs(K.cpu().numpy() - Kw)) < REL * np.max(np.abs(Jw))
