@@ -15,7 +15,7 @@
 //      number of passing kets of each bra pair is a prefix length (binary search),
 //      prefix-summed into the launch's flat quartet range.
 //   5. lai_jk_build: one launch per class pair (thread-per-quartet kernels for the
-//      small classes, warp-per-quartet otherwise), then J = J' + J'^T, K = K' + K'^T.
+//      small classes, block-per-quartet otherwise), then J = J' + J'^T, K = K' + K'^T.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -338,6 +338,36 @@ int ensure_scratch(lai_engine* E, size_t doubles) {
   LAI_CUDA_TRY(E->d_scratch.alloc(doubles * sizeof(double)));
   E->scratch_doubles = doubles;
   return LAI_OK;
+}
+
+cudaError_t scratch_pool(cudaMemPool_t* out) {
+  static std::mutex m;
+  static cudaMemPool_t pool = nullptr;  // engines of one process use one device
+  std::lock_guard<std::mutex> lock(m);
+  if (!pool) {
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t made = nullptr;
+    if (cudaError_t e = cudaMemPoolCreate(&made, &props)) return e;
+    uint64_t keep = 32 << 20;
+    if (cudaError_t e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) {
+      cudaMemPoolDestroy(made);
+      return e;
+    }
+    pool = made;
+  }
+  *out = pool;
+  return cudaSuccess;
+}
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  cudaMemPool_t pool = nullptr;
+  if (cudaError_t e = scratch_pool(&pool)) return e;
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
 namespace {
@@ -1037,6 +1067,8 @@ int create_engine(const lai_basis* basis, std::unique_ptr<lai_basis> merged, con
   E->thr = o.schwarz_threshold;
   E->prim_eps = o.prim_threshold < 0.0 ? 1e-3 * o.schwarz_threshold : o.prim_threshold;
   LAI_CUDA_TRY(cudaDeviceGetAttribute(&E->num_sms, cudaDevAttrMultiProcessorCount, o.device));
+  cudaMemPool_t pool = nullptr;
+  LAI_CUDA_TRY(scratch_pool(&pool));
   if (int rc = acquire_lanes(E->lanes)) return rc;
   E->stream = E->lanes.main;
   E->ev0 = E->lanes.t0;

@@ -45,6 +45,13 @@ struct DevBuf {
   template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Stream-ordered scratch of one call (cudaFreeAsync gives it back), from a memory pool of
+// this library that keeps up to 32 MB: the default pool returns its memory at every
+// synchronization, and an allocation after one takes 0.3 - 2 ms.  lai_engine_create makes
+// the pool, so that no call under stream capture does.
+cudaError_t scratch_pool(cudaMemPool_t* out);
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+
 template <typename T>
 cudaError_t upload(DevBuf& b, const std::vector<T>& v) {
   cudaError_t e = b.alloc(v.size() * sizeof(T));

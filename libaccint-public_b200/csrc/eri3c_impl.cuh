@@ -68,8 +68,11 @@ __global__ void __launch_bounds__(128) eri3c_kernel(Eri3cArgs g) {
     const double al = __ldg(g.exps + A.poff + ia), ca = __ldg(g.coefs + A.poff + ia);
     for (int ib = 0; ib < B.np; ++ib) {
       const double be = __ldg(g.exps + B.poff + ib), cb = __ldg(g.coefs + B.poff + ib);
-      const double p = al + be, ip = 1.0 / p;
-      const double cab = ca * cb * exp(-al * be * ip * r2);
+      const double p = al + be, ip = 1.0 / p, arg = al * be * ip * r2;
+      // exp(-80) = 2e-35: no element can show it (tight functions of two atoms, half of the
+      // primitive pairs of a cluster; the pair is the same for nearly all of a warp)
+      if (arg > 80.0) continue;
+      const double cab = ca * cb * exp(-arg);
       const double Pv[3] = {(al * A.x + be * B.x) * ip, (al * A.y + be * B.y) * ip, (al * A.z + be * B.z) * ip};
       const double PA[3] = {Pv[0] - A.x, Pv[1] - A.y, Pv[2] - A.z};
       const double PC[3] = {Pv[0] - P.x, Pv[1] - P.y, Pv[2] - P.z};

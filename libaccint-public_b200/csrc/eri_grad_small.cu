@@ -1,7 +1,7 @@
 // Dispatch of the thread-per-quartet gradient kernels (eri_grad_small.cuh) over
 // the classes they cover: the canonical (la,lb|lc,ld) with l <= 2 whose Cartesian
-// block has at most 54 components (the rest run on the warp kernel of
-// eri_grad.cu).  The kernels are instantiated in eri_grad_small_i*.cu.
+// block has at most 54 components (the rest run on the block kernel of
+// eri_grad_block.cu).  The kernels are instantiated in eri_grad_small_i*.cu.
 #include "eri_grad_small.cuh"
 
 namespace lai {

@@ -2,7 +2,7 @@
 // momentum classes: one thread per canonical quartet, everything in registers,
 // compile-time specialised on (la,lb|lc,ld) and on the derivative centre.
 //
-// Same mathematics as eri_grad.cu (d/dA_x phi_a = 2 alpha phi_{a+1x} - a_x
+// Same mathematics as eri_grad_block_impl.cuh (d/dA_x phi_a = 2 alpha phi_{a+1x} - a_x
 // phi_{a-1x}, the D centre by translational invariance), arranged like the J/K
 // kernels: the primitive loop only accumulates contracted (e0|f0)-type blocks,
 //   W[e][f] = sum_prim 2 kappa sum_r w_r pref Ix Iy Iz  over the raised shells,

@@ -67,7 +67,7 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
   const size_t bytes = sizeof(double) * stride * lai::kGradCopies;
   StreamBuf copies;
   copies.s = stream_of_call;
-  LAI_CUDA_TRY(cudaMallocAsync(&copies.p, bytes, stream_of_call));
+  LAI_CUDA_TRY(scratch_alloc(&copies.p, bytes, stream_of_call));
   double* const acc = static_cast<double*>(copies.p);
   LAI_CUDA_TRY(cudaMemsetAsync(acc, 0, bytes, stream_of_call));
   const int nbf = (int)engine->basis->nbf;

@@ -77,9 +77,14 @@ class DFFockBuilder:
             T = torch.empty((n * n, naux), dtype=torch.float64, device=self.dev)
             _lib.check(_lib.lib().lai_eri3c_device(self.engine._h, self.aux.handle(),
                                                    ctypes.c_void_p(T.data_ptr()), ctypes.c_void_p(s.cuda_stream)))
-            # B^T = L^-1 T^T  (naux x n^2)
-            self.BT = torch.linalg.solve_triangular(L, T.T, upper=False).reshape(naux, n, n).contiguous()
+            # B^T = L^-1 T^T over the pairs mu >= nu (T and B are symmetric in them, and the
+            # solve is the largest step), then both triangles (naux x n x n)
+            i, j = torch.tril_indices(n, n, device=self.dev)
+            half = torch.linalg.solve_triangular(L, T.index_select(0, i * n + j).T, upper=False)
             del T
+            k = torch.arange(n, device=self.dev)
+            hi, lo = torch.maximum(k[:, None], k), torch.minimum(k[:, None], k)
+            self.BT = half.index_select(1, (hi * (hi + 1) // 2 + lo).reshape(-1)).reshape(naux, n, n)
             e1.record(s)
             e1.synchronize()
             self.init_ms = e0.elapsed_time(e1)

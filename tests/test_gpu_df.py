@@ -95,3 +95,28 @@ def test_df_rhf_close_to_four_center(lai):
     assert r4.converged and rd.converged
     # the fitting error of the built-in cc-pVDZ-RI set: a few mHa at most
     assert abs(rd.total_energy - r4.total_energy) < 1e-2
+
+
+@pytest.mark.parametrize("R", [0.9, 4.0, 9.0, 30.0])
+def test_distant_pairs_and_half_solve(lai, oracle, R):
+    """Two atoms R bohr apart: none, some and all of the primitive pairs between them
+    below exp(-80), which the kernel leaves out (2e-35 of an element of order one), and
+    the fitted tensor, solved over the pairs mu >= nu, against the solve over all."""
+    import torch
+    Z, xyz = np.array([8, 1]), np.array([[0.0, 0.1, -0.2], [0.3, 0.0, R]])
+    b = lai.BasisSet.from_atoms(Z, xyz, "cc-pvdz")
+    aux = lai.BasisSet.from_atoms(Z, xyz, "cc-pvdz-ri")
+    eng = lai.Engine(b)
+    T, V = _dev_ints(lai, eng, aux)
+    To, Vo = oracle.orc_eri3c(b, aux), oracle.orc_eri2c(aux)
+    assert np.max(np.abs(T - To)) < 1e-12 * max(1.0, np.max(np.abs(To)))
+    df = lai.df.DFFockBuilder(eng, aux)
+    df.initialize()
+    n, na = b.nbf, aux.nbf
+    L = torch.linalg.cholesky(torch.from_numpy(0.5 * (V + V.T)).cuda())
+    full = torch.linalg.solve_triangular(L, torch.from_numpy(T.reshape(n * n, na)).cuda().T, upper=False)
+    # both solves are backward stable: cond(L) * na * eps bounds what they may differ by
+    cond = float(torch.linalg.cond(L))
+    bound = cond * na * 2.3e-16 * float(full.abs().max())
+    assert float((df.BT.reshape(na, -1) - full).abs().max()) < bound
+    assert torch.equal(df.BT, df.BT.transpose(1, 2))
