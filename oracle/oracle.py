@@ -1,7 +1,7 @@
 """Test infrastructure only: Python access to the two CPU checkers.
 
 * ``restatement()`` -- liboracle.so, the plain-C restatement of the reference
-  algorithm in rys_oracle.c (binary128 Rys roots, double ERIs, serial 8-fold
+  algorithm in rys_oracle.c (binary128 Rys roots, double ERIs, 8-fold
   symmetric J/K).  Built by ``make -C oracle restatement`` (no reference tree needed).
 * ``reference()``   -- _ref/libref_oracle.so, the UNMODIFIED reference CPU code
   compiled from its own sources by oracle/Makefile, behind ref_shim.cpp.  None when
@@ -49,8 +49,9 @@ def restatement():
         L.orc_basis_quartets.argtypes = [_I, _P, _P, _P, _P, _P, _L, _P, _P]
         L.orc_jk_list.argtypes = [_I, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P]
         L.orc_schwarz.argtypes = [_I, _P, _P, _P, _P, _P, _P]
-        L.orc_jk_sym.argtypes = [_I, _P, _P, _P, _P, _P, _P, _P, _P, _D]
-        L.orc_jk_sym.restype = ctypes.c_long
+        L.orc_canonical.argtypes = [_I, _P, _D, _P]
+        L.orc_canonical.restype = ctypes.c_long
+        L.orc_jk_values.argtypes = [_I, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P]
         L.orc_one_electron.argtypes = [_I, _P, _P, _P, _P, _P, _I, _I, _P, _P, _P]
         L.orc_eri3c.argtypes = [_I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P]
         L.orc_eri2c.argtypes = [_I, _P, _P, _P, _P, _P, _P]
@@ -208,17 +209,42 @@ def normalized_arrays(basis):
     return l, nprim, centers, exps, out
 
 
+_jk_last = None  # (key, quartets, blocks) of the last basis: an SCF asks for one J/K per iteration
+_JK_KEEP = 1 << 24  # integrals kept
+
+
 def orc_jk(basis, D, thr=1e-12):
+    """J and K by the canonical screened loop with the 8-fold symmetric scatter, and the
+    number of canonical quartets.  The blocks are computed in parallel and added in the
+    loop's order, so that the result does not depend on the number of threads."""
+    global _jk_last
     O = restatement()
     l, nprim, centers, exps, coefs = normalized_arrays(basis)
     n = basis.nbf
     D = np.ascontiguousarray(D, dtype=np.float64)
     J = np.zeros((n, n))
     K = np.zeros((n, n))
-    nq = O.orc_jk_sym(len(l), l.ctypes.data, nprim.ctypes.data, centers.ctypes.data,
-                      exps.ctypes.data, coefs.ctypes.data, D.ctypes.data, J.ctypes.data,
-                      K.ctypes.data, float(thr))
-    return J, K, nq
+    key = (float(thr), *(x.tobytes() for x in (l, nprim, centers, exps, coefs)))
+    if _jk_last is not None and _jk_last[0] == key:
+        q, parts = _jk_last[1], [(0, len(_jk_last[1]), _jk_last[2])]
+    else:
+        Q = orc_schwarz(basis)
+        q = np.zeros((O.orc_canonical(len(l), Q.ctypes.data, float(thr), None), 4), dtype=np.int32)
+        O.orc_canonical(len(l), Q.ctypes.data, float(thr), q.ctypes.data)
+        nc = (l + 1) * (l + 2) // 2
+        last = np.cumsum(nc[q].prod(axis=1, dtype=np.int64))
+        if len(q) and last[-1] <= _JK_KEEP:
+            _jk_last = (key, q, orc_quartets(basis, q))
+            parts = [(0, len(q), _jk_last[2])]
+        else:  # pieces of about _JK_KEEP integrals
+            cuts = [0, *np.flatnonzero(np.diff(last // _JK_KEEP)) + 1, len(q)]
+            parts = ((a, b, orc_quartets(basis, q[a:b])) for a, b in zip(cuts, cuts[1:]) if b > a)
+    for a, b, values in parts:
+        qs = np.ascontiguousarray(q[a:b])
+        O.orc_jk_values(len(l), l.ctypes.data, nprim.ctypes.data, centers.ctypes.data, exps.ctypes.data,
+                        coefs.ctypes.data, D.ctypes.data, len(qs), qs.ctypes.data, values.ctypes.data,
+                        J.ctypes.data, K.ctypes.data)
+    return J, K, len(q)
 
 
 def orc_quartet(basis, i, j, k, m):

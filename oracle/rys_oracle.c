@@ -408,8 +408,9 @@ int orc_schwarz(int n, const int *l, const int *nprim, const double *ctr, const 
                 const double *coefs, double *Q) {
     basis_t b;
     basis_init(&b, n, l, nprim, ctr, exps, coefs);
-    double *buf = malloc(sizeof(double) * 28 * 28 * 28 * 28);
-    for (int i = 0; i < n; ++i)
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int i = 0; i < n; ++i) {
+        double *buf = malloc(sizeof(double) * 28 * 28 * 28 * 28);
         for (int j = i; j < n; ++j) {
             quartet(&b, i, j, i, j, buf);
             const int ni = ncart(l[i]), nj = ncart(l[j]);
@@ -421,7 +422,8 @@ int orc_schwarz(int n, const int *l, const int *nprim, const double *ctr, const 
                 }
             Q[i * n + j] = Q[j * n + i] = sqrt(mx);
         }
-    free(buf);
+        free(buf);
+    }
     basis_free(&b);
     return 0;
 }
@@ -473,33 +475,38 @@ static void scatter_sym(const basis_t *b, const int *l, long nbf, int i, int j, 
                 }
 }
 
-/* Canonical screened loop + 8-fold symmetric scatter (serial).  D symmetric,
-   row-major nbf x nbf; J and K are overwritten.  Returns the number of
-   canonical quartets computed. */
-long orc_jk_sym(int n, const int *l, const int *nprim, const double *ctr, const double *exps,
-                const double *coefs, const double *D, double *J, double *K, double thr) {
-    basis_t b;
-    basis_init(&b, n, l, nprim, ctr, exps, coefs);
-    const long nbf = b.foff[n];
-    double *Q = malloc(sizeof(double) * n * n);
-    orc_schwarz(n, l, nprim, ctr, exps, coefs, Q);
-    double *g = malloc(sizeof(double) * 28 * 28 * 28 * 28);
-    memset(J, 0, sizeof(double) * nbf * nbf);
-    memset(K, 0, sizeof(double) * nbf * nbf);
+/* Canonical screened quartets of the 8-fold symmetric loop, in its order: writes
+   q[4t..4t+3] when q is not NULL and returns their number. */
+long orc_canonical(int n, const double *Q, double thr, int *q) {
     long count = 0;
     for (int i = 0; i < n; ++i)
         for (int j = i; j < n; ++j)
             for (int k = i; k < n; ++k)
                 for (int m = (k == i ? j : k); m < n; ++m) {
                     if (Q[i * n + j] * Q[k * n + m] < thr) continue;
-                    quartet(&b, i, j, k, m, g);
+                    if (q) {
+                        int *x = q + 4 * count;
+                        x[0] = i; x[1] = j; x[2] = k; x[3] = m;
+                    }
                     ++count;
-                    scatter_sym(&b, l, nbf, i, j, k, m, g, D, J, K);
                 }
-    free(g);
-    free(Q);
-    basis_free(&b);
     return count;
+}
+
+/* J/K contributions of listed canonical quartets whose blocks are `values`
+   (orc_basis_quartets), ADDED to J and K in the order of the list. */
+void orc_jk_values(int n, const int *l, const int *nprim, const double *ctr, const double *exps,
+                   const double *coefs, const double *D, long nq, const int *q, const double *values,
+                   double *J, double *K) {
+    basis_t b;
+    basis_init(&b, n, l, nprim, ctr, exps, coefs);
+    const long nbf = b.foff[n];
+    for (long t = 0; t < nq; ++t) {
+        const int *x = q + 4 * t;
+        scatter_sym(&b, l, nbf, x[0], x[1], x[2], x[3], values, D, J, K);
+        values += (long)ncart(l[x[0]]) * ncart(l[x[1]]) * ncart(l[x[2]]) * ncart(l[x[3]]);
+    }
+    basis_free(&b);
 }
 
 /* ------------------------------------------------------------------------- */
