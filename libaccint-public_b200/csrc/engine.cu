@@ -476,6 +476,7 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
   const bool untuned = tune.ps == 0 && tune.ksuper == 0 && tune.kernel == lai::KERNEL_DEFAULT;
   if (untuned && !fp32 && args.mode == lai::MODE_JK && lai::block_for_few(blk, E->num_sms)) tune.kernel = lai::KERNEL_BLOCK;
   if (lai::small_class_supported(la, lb, lc, ld) && tune.kernel != lai::KERNEL_BLOCK) {
+    fp32 = fp32 && lai::small_fp32_class(la, lb, lc, ld);
     const int rc = lai::launch_small(blk, args, E->tab, E->stream, fp32, E->num_sms, tune);
     if (ran_fp32) *ran_fp32 = fp32;
     if (rc < 0) return fail(LAI_ECUDA, std::string("small-class launch failed: ") +

@@ -58,10 +58,11 @@ int launch_blockq(const QuartetBlock& blk, const JKArgs& args, const RysTablesVi
 
 int block_ket_chunks(int lc, int ld) { return ncart(lc) / block_detail::chunk_components(lc, ld); }
 
-// FP32 covers the d and f classes with at most 1152 contracted (e0|f0) integrals; the
-// larger ones, and the g classes, run in FP64 in a mixed-precision build.
+// FP32 covers the d and f classes with at most 1024 contracted (e0|f0) integrals: up to
+// (dd|dd), 961.  The larger ones, from (fd|fp) with 1150 on, and the g classes run in FP64
+// in a mixed-precision build.
 bool block_fp32_class(int la, int lb, int lc, int ld) {
-  return la <= 3 && ncart_range(la, la + lb) * ncart_range(lc, lc + ld) <= 1152;
+  return la <= 3 && ncart_range(la, la + lb) * ncart_range(lc, lc + ld) <= 1024;
 }
 
 // Launches of the thread-per-quartet classes with three roots or more and few quartets:

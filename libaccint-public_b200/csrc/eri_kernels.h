@@ -38,6 +38,9 @@ int launch_small_list(int la, int lb, int lc, int ld, const MultiEntry* list, in
 int launch_small(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,
                  cudaStream_t stream, bool fp32, int num_sms, LaunchTune tune = LaunchTune{});
 bool small_class_supported(int la, int lb, int lc, int ld);
+// Whether the class has an FP32 variant.  Of the g classes only (gs|ss) has: the FP32
+// primitive sums are compensated up to 18 (e0|f0) integrals, and (gs|ps) has 45.
+constexpr bool small_fp32_class(int la, int lb, int lc, int ld) { return la <= 3 || lb + lc + ld == 0; }
 
 // Bra-sliced kernels for the medium classes (eri_sliced.cu); same return codes.
 int launch_sliced(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,

@@ -813,18 +813,19 @@ __global__ void __launch_bounds__(256, (small_min_blocks<LA, LB, LC, LD, R>()))
 
 namespace small_detail {
 
-// The kernel of a variant (0: FP64, 1: FP64 split, 2: FP32, 3: FP32 split) and its
-// resident blocks per SM; -3 on a CUDA error.  Separate instantiations keep the unsplit
+// The kernel of a variant (0: FP64, 1: FP64 split, 2: FP32, 3: FP32 split; FP64 for both in
+// a class without FP32) and its resident blocks per SM; -3 on a CUDA error.  Separate instantiations keep the unsplit
 // kernel's register allocation independent of the split one.
 using SmallKernel = void (*)(QuartetBlock, JKArgs, RysTablesView, int, int, const MultiEntry*, int, int64_t);
 constexpr int kSmallThreads = 256;
 template <int LA, int LB, int LC, int LD>
 int small_variant(int v, SmallKernel* kern, size_t* smem) {
+  using Low = std::conditional_t<small_fp32_class(LA, LB, LC, LD), float, double>;
   const SmallKernel kerns[4] = {
       eri_small_kernel<LA, LB, LC, LD, double, false>, eri_small_kernel<LA, LB, LC, LD, double, true>,
-      eri_small_kernel<LA, LB, LC, LD, float, false>, eri_small_kernel<LA, LB, LC, LD, float, true>};
+      eri_small_kernel<LA, LB, LC, LD, Low, false>, eri_small_kernel<LA, LB, LC, LD, Low, true>};
   *kern = kerns[v];
-  *smem = v >= 2 ? small_table_bytes<LA, LB, LC, LD, float>() : small_table_bytes<LA, LB, LC, LD, double>();
+  *smem = v >= 2 ? small_table_bytes<LA, LB, LC, LD, Low>() : small_table_bytes<LA, LB, LC, LD, double>();
   static std::atomic<int> per_sm[4];
   int n = per_sm[v].load(std::memory_order_relaxed);
   if (n == 0) {
