@@ -388,21 +388,6 @@ void destroy_lanes(LaneSet& set) {
 }
 }  // namespace
 
-// The first n - 1 side streams (and their events) of the set.
-int extend_lanes(LaneSet& set, size_t n) {
-  while (set.ev.size() < n) {
-    cudaEvent_t e = nullptr;
-    LAI_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    set.ev.push_back(e);
-  }
-  while (set.side.size() + 1 < n) {
-    cudaStream_t s = nullptr;
-    LAI_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    set.side.push_back(s);
-  }
-  return LAI_OK;
-}
-
 int acquire_lanes(LaneSet& out) {
   {
     std::lock_guard<std::mutex> lock(g_lane_mutex);
@@ -412,7 +397,16 @@ int acquire_lanes(LaneSet& out) {
       return LAI_OK;
     }
   }
-  if (int rc = extend_lanes(out, kLanes)) return rc;
+  while (out.ev.size() < (size_t)kLanes) {
+    cudaEvent_t e = nullptr;
+    LAI_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    out.ev.push_back(e);
+  }
+  while (out.side.size() + 1 < (size_t)kLanes) {
+    cudaStream_t s = nullptr;
+    LAI_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    out.side.push_back(s);
+  }
   LAI_CUDA_TRY(cudaStreamCreateWithFlags(&out.main, cudaStreamNonBlocking));
   LAI_CUDA_TRY(cudaEventCreate(&out.t0));
   LAI_CUDA_TRY(cudaEventCreate(&out.t1));
@@ -755,7 +749,7 @@ int build_launches(lai_engine* E) {
 // J' = K' = 0 and every class-pair launch of a build of the density dD, on `stream`
 // (spread over the lanes).  Part 1 of a mixed build's blocks runs in FP32.
 int enqueue_jk(lai_engine* E, const double* dD, cudaStream_t stream, const lai_jk_opts& o, double cut, bool timed,
-               lai_jk_report& rep, size_t nlanes = kLanes) {
+               lai_jk_report& rep) {
   const int nbf = (int)E->basis->nbf;
   const bool batched = E->nsys > 1;
   const size_t elems = engine_mat_elems(E);
@@ -803,7 +797,7 @@ int enqueue_jk(lai_engine* E, const double* dD, cudaStream_t stream, const lai_j
   }
   E->prof_n = 0;
   // profiled builds time every launch by itself, in block order on one stream
-  LaunchLanes lanes(E, stream, o.profile ? 1 : nlanes);
+  LaunchLanes lanes(E, stream, o.profile ? 1 : kLanes);
   if (!o.profile && !mixed && o.shard_count == 1 && !E->tuned) {
     for (const auto& it : E->launches) {
       LAI_CUDA_TRY(lanes.pick(it.work, &E->stream));
@@ -871,50 +865,6 @@ int enqueue_jk(lai_engine* E, const double* dD, cudaStream_t stream, const lai_j
   return LAI_OK;
 }
 
-// The engine's build plan for these options, captured as a graph over the engine's own
-// copy of the density; *plan = nullptr where none is used.  The smallest builds are bound by
-// the issue of their launches, forks and joins: H2O/STO-3G, 6 launches, 50.7 -> 38.2 us a
-// build with the graph, (H2O)5/6-31G 333 -> 324 us, larger ones the same.  The plan is made
-// at the second build with the same options (a one-shot build would only pay for it) and
-// dropped with any buffer it points into; none above kPlanElems matrix elements, where the
-// copy of the density is no longer negligible.
-constexpr size_t kPlanElems = size_t(1) << 20;
-int build_plan(lai_engine* E, cudaStream_t stream, const lai_jk_opts& o, double cut, lai_engine::Plan** plan) {
-  *plan = nullptr;
-  const size_t elems = engine_mat_elems(E);
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (o.profile || elems == 0 || elems > kPlanElems ||
-      cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-    return LAI_OK;
-  lai_engine::Plan& p = E->plan;
-  if (!p.matches(o, cut)) {
-    p.release();
-    p.cut = cut;
-    p.shard_index = o.shard_index;
-    p.shard_count = o.shard_count;
-    p.fp32_prim_rel = o.fp32_prim_rel;
-    p.seen = true;
-    return LAI_OK;
-  }
-  if (!p.exec) {
-    if (E->d_plan_D.bytes < sizeof(double) * elems) LAI_CUDA_TRY(E->d_plan_D.alloc(sizeof(double) * elems));
-    std::lock_guard<std::recursive_mutex> lock(E->lanes_mutex);
-    cudaGraph_t graph = nullptr;
-    cudaStream_t own = E->lanes.main;
-    if (int rc = extend_lanes(E->lanes, kPlanLanes)) return rc;
-    LAI_CUDA_TRY(cudaStreamBeginCapture(own, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_jk(E, E->d_plan_D.as<double>(), own, o, cut, false, p.report, kPlanLanes);
-    const cudaError_t ce = cudaStreamEndCapture(own, &graph);
-    cudaError_t ie = ce;
-    if (!rc && ce == cudaSuccess) ie = cudaGraphInstantiate(&p.exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
-    if (rc) return rc;
-    LAI_CUDA_TRY(ie);
-  }
-  *plan = &p;
-  return LAI_OK;
-}
-
 // forced_cut >= 0: use this Schwarz cut for the FP32 split instead of deriving it
 // from max|D| (which synchronizes the stream; not allowed while capturing a graph).
 int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t stream,
@@ -938,18 +888,8 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
   }
   if (cut > 0.0)
     if (int rc = build_split(E, cut)) return rc;
-  lai_engine::Plan* plan = nullptr;
-  if (int rc = build_plan(E, stream, o, cut, &plan)) return rc;
   lai_jk_report r{};
-  if (plan) {
-    if (timed) LAI_CUDA_TRY(cudaEventRecord(E->ev0, stream));
-    LAI_CUDA_TRY(cudaMemcpyAsync(E->d_plan_D.p, dD, sizeof(double) * elems, cudaMemcpyDeviceToDevice, stream));
-    LAI_CUDA_TRY(cudaGraphLaunch(plan->exec, stream));
-    r = plan->report;
-    E->prof_n = 0;
-  } else if (int rc = enqueue_jk(E, dD, stream, o, cut, timed, r)) {
-    return rc;
-  }
+  if (int rc = enqueue_jk(E, dD, stream, o, cut, timed, r)) return rc;
   const int64_t nn = (int64_t)elems;
   if (nn > 0) {
     if (batched)

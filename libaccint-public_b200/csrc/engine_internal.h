@@ -94,7 +94,6 @@ struct LaneSet {
   cudaEvent_t t0 = nullptr, t1 = nullptr;  // timed builds
 };
 constexpr int kLanes = 8;
-constexpr int kPlanLanes = 32;  // branches of a captured build (a graph's are not bound to hardware queues)
 constexpr size_t kPooledLaneSets = 4;
 int acquire_lanes(LaneSet& out);
 void release_lanes(LaneSet& set);
@@ -209,28 +208,9 @@ struct lai_engine {
   cudaGraphExec_t graph_exec = nullptr;
   GraphKey graph_key{};
   lai_jk_report graph_report{};
-  // The launches of a build as a graph over d_plan_D, for one set of options (build_plan).
-  struct Plan {
-    cudaGraphExec_t exec = nullptr;
-    bool seen = false;
-    double cut = 0.0, fp32_prim_rel = 0.0;
-    int shard_index = 0, shard_count = 1;
-    lai_jk_report report{};
-    bool matches(const lai_jk_opts& o, double c) const {
-      return seen && cut == c && shard_index == o.shard_index && shard_count == o.shard_count &&
-             fp32_prim_rel == o.fp32_prim_rel;
-    }
-    void release() {
-      if (exec) cudaGraphExecDestroy(exec);
-      exec = nullptr;
-      seen = false;
-    }
-  } plan;
-  lai::host::DevBuf d_plan_D;
   void release_graph() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     graph_exec = nullptr;
-    plan.release();
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // per-launch profile of the last build with opts.profile
@@ -241,7 +221,7 @@ struct lai_engine {
   int prof_n = 0;
   // streams the independent class-pair launches of one build are spread over
   lai::host::LaneSet lanes;
-  std::recursive_mutex lanes_mutex;   // held while launches are queued on the lanes, or captured
+  std::mutex lanes_mutex;             // held while launches are queued on the lanes
   cudaStream_t fork_stream = nullptr; // caller's stream while a build is spread over lanes
   std::vector<int> launch_order;      // blocks by descending estimated work
   // The launches of a plain build (FP64, one shard, untuned), by descending estimated
@@ -304,7 +284,7 @@ class LaunchLanes {
   std::vector<double> load_;   // estimated work per lane; < 0: not forked yet
   // calls of several threads on one engine queue their launches one after another (they
   // share the lanes' events)
-  std::unique_lock<std::recursive_mutex> lock_;
+  std::unique_lock<std::mutex> lock_;
 };
 double alg_work(int la, int lb, int lc, int ld, int Ka, int Kb, int Kc, int Kd);
 double alg_per_prim(int la, int lb, int lc, int ld);

@@ -1,7 +1,8 @@
-"""Repeated builds (captured at the second one with the same options) against the first,
-with options and densities that change in between, on several streams, and inside a
-caller's own capture."""
+"""Repeated builds against the first, with options and densities that change in between, on
+several streams, and inside a caller's own capture; and what each of the first builds costs."""
 import importlib
+import statistics
+import time
 
 import numpy as np
 import pytest
@@ -65,3 +66,29 @@ def test_build_inside_a_callers_capture():
         torch.cuda.synchronize()
         assert np.max(np.abs(J.cpu().numpy() - Jw)) < REL * np.max(np.abs(Jw))
         assert np.max(np.abs(K.cpu().numpy() - Kw)) < REL * np.max(np.abs(Jw))
+
+
+def test_no_build_but_the_first_prepares():
+    """The second build of an engine costs what the later ones do, in time and in device
+    memory (666 launches of H2O/cc-pVQZ: work of its own would show)."""
+    import torch
+    w = lai.workloads.make("h2o1_ccpvqz")
+    stream = torch.cuda.Stream()
+    second, later = [], []
+    for _ in range(3):
+        eng = lai.Engine(w.basis)
+        d = torch.from_numpy(w.D).cuda()
+        J, K = torch.empty_like(d), torch.empty_like(d)
+        ms, free = [], []
+        for _ in range(8):
+            torch.cuda.synchronize()
+            free.append(torch.cuda.mem_get_info()[0])
+            t = time.perf_counter()
+            eng.jk_device(d.data_ptr(), J.data_ptr(), K.data_ptr(), stream=stream.cuda_stream)
+            torch.cuda.synchronize()
+            ms.append(1e3 * (time.perf_counter() - t))
+        second.append(ms[1])
+        later.append(statistics.median(ms[2:]))
+        assert len(set(free[1:])) == 1, free
+        eng.close()
+    assert min(second) < 1.3 * min(later), (second, later)
