@@ -682,13 +682,14 @@ def main():
 
     # set-up, outside the timed region: the project's autotuner times each
     # class-pair launch under its kernel families and launch shapes on this
-    # density and keeps the fastest (every rank tunes its own engine)
+    # density and keeps the fastest where whole builds gain (every rank tunes its own engine)
     tune = None
     if not args.no_autotune:
         t0 = time.perf_counter()
         tb, ta = eng.autotune(D.data_ptr(), stream=stream.cuda_stream)
         torch.cuda.synchronize()
-        tune = {"seconds": time.perf_counter() - t0, "launch_ms_before": tb, "launch_ms_after": ta}
+        tune = {"seconds": time.perf_counter() - t0, "launch_ms_before": tb, "launch_ms_after": ta,
+                "kept": bool(eng.tune_table()[:, 7:9].any())}
 
     def step(profile=False):
         rep = eng.jk_device(D.data_ptr(), J.data_ptr(), K.data_ptr(), stream=stream.cuda_stream,
@@ -823,7 +824,8 @@ def main():
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": jk_config(args, w, total_q, ws),
-            "schedule": "autotuned in the set-up (lai_engine_autotune)" if tune else "built-in launch heuristics",
+            "schedule": "autotuned in the set-up (lai_engine_autotune)" if tune and tune["kept"]
+            else "built-in launch heuristics",
             "jk_build_s": ms_per_step * 1e-3,
             "energy": E, "energy_e2e": E2,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 8 * n * n,

@@ -362,10 +362,13 @@ LAI_API int64_t lai_engine_quartet_count(lai_engine* engine);
 /* Autotuner: times every thread-per-quartet class launch of the engine under a
  * few launch configurations (lanes per quartet 1..8, chunks per super-chunk 1, 4,
  * 16), and every other class launch under each kernel family that covers it
- * (block-per-quartet, bra-sliced, tiled), on the device density d_D, and keeps the
- * fastest for later builds.
- * ms_before/ms_after (may be NULL): summed launch times with the built-in
- * heuristic and with the chosen configurations.  Synchronizes `stream`. */
+ * (block-per-quartet, bra-sliced, tiled), on the device density d_D.  Later builds use
+ * the fastest of them if a whole build is faster with them than with the built-in
+ * schedule, which runs launches side by side and groups the small ones; otherwise, and
+ * after an error, the engine is as before.
+ * ms_before/ms_after (may be NULL): summed times of the launches, one at a time, with the
+ * built-in heuristic and with the configurations that later builds use.  Synchronizes
+ * `stream`. */
 LAI_API int lai_engine_autotune(lai_engine* engine, const double* d_D, void* stream, double* ms_before,
                                 double* ms_after);
 /* The launch table: per class-pair block, 10 ints: la, lb, lc, ld, bra and ket

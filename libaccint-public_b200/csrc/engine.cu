@@ -910,6 +910,118 @@ int run_jk(lai_engine* E, const double* dD, double* dJ, double* dK, cudaStream_t
   return LAI_OK;
 }
 
+// Launch choices of every block, timed one launch at a time, and whether builds use them.
+int tune_blocks(lai_engine* engine, const double* d_D, cudaStream_t s, double* ms_before, double* ms_after) {
+  const size_t elems = engine_mat_elems(engine);
+  const int copies = accumulator_copies(elems);
+  lai::JKArgs args{};
+  args.D = d_D;
+  args.J = engine->jp();
+  args.K = engine->kp(copies * elems);
+  args.copy_mask = copies - 1;
+  args.copy_stride = (int64_t)elems;
+  args.nbf = (int)engine->basis->nbf;
+  args.mode = lai::MODE_JK;
+  args.prim_eps = engine->prim_eps;
+  if (engine->nsys > 1) {
+    args.sys_off = engine->d_sys_off.as<int64_t>();
+    args.sys_nbf = engine->d_sys_nbf.as<int>();
+  }
+  struct Events {
+    cudaEvent_t e[2] = {nullptr, nullptr};
+    ~Events() { for (auto x : e) if (x) cudaEventDestroy(x); }
+  } ev;
+  for (auto& x : ev.e)
+    if (cudaEventCreate(&x) != cudaSuccess) return LAI_ECUDA;
+  const cudaEvent_t e0 = ev.e[0], e1 = ev.e[1];
+  struct Restore {
+    lai_engine* E;
+    cudaStream_t saved;
+    ~Restore() { E->stream = saved; }
+  } restore{engine, engine->stream};
+  engine->stream = s;
+  double before = 0.0, after = 0.0;
+  auto time_launch = [&](const lai::QuartetBlock& q, lai::LaunchTune t, float* ms) -> int {
+    float best = 1e30f;
+    for (int rep = 0; rep < 2; ++rep) {  // the first run warms caches, the minimum counts
+      if (cudaEventRecord(e0, s) != cudaSuccess) return LAI_ECUDA;
+      if (int r = launch_block(engine, q, args, false, nullptr, t)) return r;
+      if (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) return LAI_ECUDA;
+      float m = 0;
+      cudaEventElapsedTime(&m, e0, e1);
+      best = std::min(best, m);
+    }
+    *ms = best;
+    return LAI_OK;
+  };
+  for (auto& bp : engine->blocks) {
+    const lai::QuartetBlock q = make_block(engine, *bp);
+    float base = 0;
+    if (const int rc = time_launch(q, bp->tune, &base)) return rc;
+    before += base;
+    if (!lai::small_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb)) {
+      // kernel family: block-per-quartet, bra-sliced, tiled
+      lai::LaunchTune best = bp->tune;
+      float best_ms = base;
+      for (int k : {lai::KERNEL_BLOCK, lai::KERNEL_SLICED, lai::KERNEL_TILED}) {
+        if (k == lai::KERNEL_SLICED && !lai::sliced_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb))
+          continue;
+        lai::LaunchTune t;
+        t.kernel = k;
+        float m = 0;
+        if (const int rc = time_launch(q, t, &m)) return rc;
+        if (m < 0.98f * best_ms) { best_ms = m; best = t; }
+      }
+      bp->tune = best;
+      after += best_ms;
+      continue;
+    }
+    const int Kab = q.bra.Ka * q.bra.Kb;
+    lai::LaunchTune best = bp->tune;
+    float best_ms = base;
+    for (int ps = 1; ps <= 8 && ps < 2 * Kab; ps <<= 1)
+      for (int ks : {1, 4, 16}) {
+        float m = 0;
+        if (const int rc = time_launch(q, lai::LaunchTune{ps, ks}, &m)) return rc;
+        if (m < 0.98f * best_ms) { best_ms = m; best = lai::LaunchTune{ps, ks}; }
+      }
+    if (q.total - q.t_begin < (int64_t)engine->num_sms * 64) {
+      float m = 0;
+      lai::LaunchTune t;
+      t.kernel = lai::KERNEL_BLOCK;
+      if (const int rc = time_launch(q, t, &m)) return rc;
+      if (m < 0.98f * best_ms) { best_ms = m; best = t; }
+    }
+    bp->tune = best;
+    after += best_ms;
+  }
+  // The launches were timed one at a time, a build runs them side by side: the choices stay
+  // only if a whole build is faster with them than with the built-in schedule.
+  float build[2] = {1e30f, 1e30f};
+  lai_jk_opts o;
+  lai_jk_opts_default(&o);
+  for (int rep = 0; rep < 3; ++rep)  // the first of each warms up
+    for (int k = 0; k < 2; ++k) {
+      engine->tuned = k == 1;
+      lai_jk_report r{};
+      if (cudaEventRecord(e0, s) != cudaSuccess) return LAI_ECUDA;
+      const int rc = enqueue_jk(engine, d_D, s, o, 0.0, false, r);
+      engine->tuned = false;
+      if (rc) return rc;
+      float m = 0;
+      if (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+          cudaEventElapsedTime(&m, e0, e1) != cudaSuccess)
+        return LAI_ECUDA;
+      if (rep > 0) build[k] = std::min(build[k], m);
+    }
+  engine->tuned = build[1] < 0.99f * build[0];
+  if (!engine->tuned)
+    for (auto& bp : engine->blocks) bp->tune = lai::LaunchTune{};
+  if (ms_before) *ms_before = before;
+  if (ms_after) *ms_after = engine->tuned ? after : before;
+  return LAI_OK;
+}
+
 // splitmix64
 inline uint64_t mix64(uint64_t& x) {
   uint64_t z = (x += 0x9E3779B97F4A7C15ull);
@@ -1346,88 +1458,13 @@ int lai_engine_autotune(lai_engine* engine, const double* d_D, void* stream, dou
   LAI_CUDA_TRY(dK.alloc(sizeof(double) * elems));
   if (int rc = run_jk(engine, d_D, dJ.as<double>(), dK.as<double>(), s, o, nullptr, false)) return rc;
   engine->release_graph();
-  engine->tuned = true;
-  cudaEvent_t e0, e1;
-  LAI_CUDA_TRY(cudaEventCreate(&e0));
-  LAI_CUDA_TRY(cudaEventCreate(&e1));
-  lai::JKArgs args{};
-  args.D = d_D;
-  args.J = engine->jp();
-  args.K = engine->kp(elems);
-  args.nbf = (int)engine->basis->nbf;
-  args.mode = lai::MODE_JK;
-  args.prim_eps = engine->prim_eps;
-  if (engine->nsys > 1) {
-    args.sys_off = engine->d_sys_off.as<int64_t>();
-    args.sys_nbf = engine->d_sys_nbf.as<int>();
+  engine->tuned = false;
+  for (auto& bp : engine->blocks) bp->tune = lai::LaunchTune{};
+  const int rc = tune_blocks(engine, d_D, s, ms_before, ms_after);
+  if (rc) {
+    for (auto& bp : engine->blocks) bp->tune = lai::LaunchTune{};
+    return fail(rc, "lai_engine_autotune: a timing launch failed");
   }
-  cudaStream_t saved = engine->stream;
-  engine->stream = s;
-  double before = 0.0, after = 0.0;
-  int rc = LAI_OK;
-  auto time_launch = [&](const lai::QuartetBlock& q, lai::LaunchTune t, float* ms) -> int {
-    float best = 1e30f;
-    for (int rep = 0; rep < 2; ++rep) {  // the first run warms caches, the minimum counts
-      if (cudaEventRecord(e0, s) != cudaSuccess) return LAI_ECUDA;
-      if (int r = launch_block(engine, q, args, false, nullptr, t)) return r;
-      if (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) return LAI_ECUDA;
-      float m = 0;
-      cudaEventElapsedTime(&m, e0, e1);
-      best = std::min(best, m);
-    }
-    *ms = best;
-    return LAI_OK;
-  };
-  for (auto& bp : engine->blocks) {
-    const lai::QuartetBlock q = make_block(engine, *bp);
-    bp->tune = lai::LaunchTune{};
-    float base = 0;
-    if ((rc = time_launch(q, bp->tune, &base))) break;
-    before += base;
-    if (!lai::small_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb)) {
-      // kernel family: block-per-quartet, bra-sliced, tiled
-      lai::LaunchTune best = bp->tune;
-      float best_ms = base;
-      for (int k : {lai::KERNEL_BLOCK, lai::KERNEL_SLICED, lai::KERNEL_TILED}) {
-        if (k == lai::KERNEL_SLICED && !lai::sliced_class_supported(q.bra.la, q.bra.lb, q.ket.la, q.ket.lb))
-          continue;
-        lai::LaunchTune t;
-        t.kernel = k;
-        float m = 0;
-        if ((rc = time_launch(q, t, &m))) break;
-        if (m < 0.98f * best_ms) { best_ms = m; best = t; }
-      }
-      if (rc) break;
-      bp->tune = best;
-      after += best_ms;
-      continue;
-    }
-    const int Kab = q.bra.Ka * q.bra.Kb;
-    lai::LaunchTune best = bp->tune;
-    float best_ms = base;
-    for (int ps = 1; ps <= 8 && ps < 2 * Kab; ps <<= 1)
-      for (int ks : {1, 4, 16}) {
-        float m = 0;
-        if ((rc = time_launch(q, lai::LaunchTune{ps, ks}, &m))) break;
-        if (m < 0.98f * best_ms) { best_ms = m; best = lai::LaunchTune{ps, ks}; }
-      }
-    if (!rc && q.total - q.t_begin < (int64_t)engine->num_sms * 64) {
-      float m = 0;
-      lai::LaunchTune t;
-      t.kernel = lai::KERNEL_BLOCK;
-      rc = time_launch(q, t, &m);
-      if (!rc && m < 0.98f * best_ms) { best_ms = m; best = t; }
-    }
-    if (rc) break;
-    bp->tune = best;
-    after += best_ms;
-  }
-  engine->stream = saved;
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (rc) return fail(rc, "lai_engine_autotune: a timing launch failed");
-  if (ms_before) *ms_before = before;
-  if (ms_after) *ms_after = after;
   return LAI_OK;
 }
 

@@ -300,7 +300,8 @@ class Engine:
 
     def autotune(self, d_D, stream=0):
         """Times each class launch under a few launch configurations on the device
-        density d_D and keeps the fastest; returns (ms_before, ms_after)."""
+        density d_D and keeps the fastest if a whole build is faster with them; returns
+        (ms_before, ms_after), the summed launch times."""
         a = ctypes.c_double()
         b = ctypes.c_double()
         _lib.check(_lib.lib().lai_engine_autotune(self._h, ctypes.c_void_p(d_D), ctypes.c_void_p(stream),
