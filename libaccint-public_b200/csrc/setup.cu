@@ -10,9 +10,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <utility>
 
 #include "engine_internal.h"
 #include "fp32_tables.h"
@@ -45,6 +47,15 @@ struct ClassTables {
   PairClassDev out;         // tables to write (FP32 copies only where not null)
   unsigned long long* qmax; // largest primitive bound of the class, as its bit pattern
 };
+
+// Pairs [pair0, pair0 + n) of the pair list, of one class, in the bounds of one stage: shell
+// pairs (0) or their primitive pairs, prim0 the first (1).
+struct Piece {
+  int stage, n;
+  int64_t pair0, prim0;
+  ClassTables tab;
+};
+constexpr size_t kBoundBytes = size_t(256) << 20;
 
 __device__ __forceinline__ int find_class(const ClassTables* __restrict__ cls, int ncls, int64_t e) {
   int lo = 0, hi = ncls;
@@ -252,9 +263,9 @@ int setup_pairs(lai_engine* E) {
     hexp.insert(hexp.end(), sh[i].exps.begin(), sh[i].exps.end());
     hcoef.insert(hcoef.end(), sh[i].coefs.begin(), sh[i].coefs.end());
   }
-  int64_t npairs = 0, nelem = 0, maxn = 0;
+  int64_t npairs = 0, nelem = 0;
   std::vector<int2> hp;
-  std::vector<ClassTables> raw(nc), one(nc);
+  std::vector<ClassTables> raw(nc);
   for (int c = 0; c < nc; ++c) {
     const auto& cl = *E->classes[c];
     const int Kab = cl.Ka * cl.Kb, n = cl.n();
@@ -264,15 +275,10 @@ int setup_pairs(lai_engine* E) {
     a.elem0 = nelem; a.pair0 = npairs; a.src0 = nelem;
     a.out.la = cl.la; a.out.lb = cl.lb; a.out.Ka = cl.Ka; a.out.Kb = cl.Kb; a.out.npairs = n;
     raw[c] = a;
-    a.Kb = a.Kab = 1; a.npairs = n * Kab; a.parentK = Kab;
-    a.out.Ka = a.out.Kb = 1; a.out.npairs = n * Kab;
-    one[c] = a;
     npairs += n;
     nelem += (int64_t)n * Kab;
-    maxn = std::max<int64_t>(maxn, (int64_t)n * Kab);
   }
-  // temporary buffers of the set-up: one allocation for the unsorted tables of one stage
-  // at a time (the one-primitive stage overwrites the contracted one)
+  // temporary buffers of the set-up
   DevBuf d_in, d_tmp, d_bounds, d_meta;
   DevShell* ds; double *de, *dcf; int2* dp; int64_t* iota64; int* iota32;
   {
@@ -300,6 +306,53 @@ int setup_pairs(lai_engine* E) {
     LAI_CUDA_TRY(cudaMemcpyAsync(d_in.p, pack.data(), pack.size(), cudaMemcpyHostToDevice, s));
     LAI_CUDA_TRY(cudaStreamSynchronize(s));
   }
+  // ---- bounds: of the shell pairs (ab|ab), and of every primitive pair run as a
+  // one-primitive pair (by the Schwarz inequality a primitive quartet contributes at most
+  // q_ab q_cd to any integral of its quartet).  Their unsorted tables, 340 bytes for each
+  // primitive pair of the basis, most of them far below the cut in a large one, are formed
+  // in pieces: ranges of a class's pairs, as many at a time as fit kBoundBytes. ----
+  std::vector<Piece> pieces;
+  for (int stage = 0; stage < 2; ++stage)
+    for (int c = nc - 1; c >= 0; --c) {
+      ClassTables a = raw[c];
+      if (stage == 1) {
+        a.parentK = a.Kab;
+        a.Kb = a.Kab = 1;
+        a.out.Ka = a.out.Kb = 1;
+      }
+      const int n = raw[c].npairs, per = stage == 0 ? 1 : raw[c].Kab;
+      const size_t pair = (size_t)raw[c].Kab * (PF_COUNT + kBraRec + kKetRec) * sizeof(double) +
+                          per * (6 * sizeof(double) + 4 * sizeof(int));
+      const int most = (int)std::max<size_t>(kKetTile, std::min<size_t>(INT_MAX / per, kBoundBytes / 2 / pair));
+      for (int p = 0; p < n; p += most) {
+        const int np = std::min(most, n - p);
+        Piece pc{stage, np, raw[c].pair0 + p, raw[c].elem0 + (int64_t)p * raw[c].Kab, a};
+        pc.tab.pair0 = pc.pair0;
+        pc.tab.npairs = pc.tab.out.npairs = np * per;
+        pieces.push_back(pc);
+      }
+    }
+  // batches [first, last) of pieces of one stage
+  std::vector<std::pair<size_t, size_t>> batches;
+  size_t need = 0, batch_pieces = 0;
+  int64_t maxn = 0;
+  for (size_t i = 0; i < pieces.size();) {
+    Layout L;
+    size_t j = i;
+    while (j < pieces.size() && pieces[j].stage == pieces[i].stage) {
+      Layout next = L;
+      PairClassDev v = pieces[j].tab.out;
+      lay_out_class(next, v, false);
+      if (j > i && next.at > kBoundBytes) break;
+      L = next;
+      maxn = std::max<int64_t>(maxn, pieces[j].tab.npairs);
+      ++j;
+    }
+    need = std::max(need, L.at);
+    batch_pieces = std::max(batch_pieces, j - i);
+    batches.emplace_back(i, j);
+    i = j;
+  }
   double *d_q, *d_qprim;
   {
     Layout L;
@@ -316,44 +369,39 @@ int setup_pairs(lai_engine* E) {
     }
   }
   iota_kernel<<<blocks_for(maxn + 1), 256, 0, s>>>(iota64, iota32, maxn);
-
-  // ---- bounds: of the shell pairs (ab|ab), and of every primitive pair run as a
-  // one-primitive pair (by the Schwarz inequality a primitive quartet contributes at most
-  // q_ab q_cd to any integral of its quartet) ----
-  size_t need = 0;
-  for (auto* v : {&raw, &one}) {
-    Layout L;
-    for (auto& c : *v) lay_out_class(L, c.out, false);
-    need = std::max(need, L.at);
-  }
   LAI_CUDA_TRY(d_tmp.alloc(need));
-  LAI_CUDA_TRY(d_meta.alloc(sizeof(ClassTables) * nc));
-  for (int stage = 0; stage < 2; ++stage) {
-    auto& v = stage == 0 ? raw : one;
+  LAI_CUDA_TRY(d_meta.alloc(sizeof(ClassTables) * batch_pieces));
+  for (const auto& [first, last] : batches) {
     Layout L;
     L.base = d_tmp.as<char>();
-    for (auto& c : v) {
-      lay_out_class(L, c.out, false);
-      if (int rc = clear_ket_pads(c.out, s)) return rc;
+    std::vector<ClassTables> meta;
+    int64_t elems = 0;
+    for (size_t i = first; i < last; ++i) {
+      ClassTables& t = pieces[i].tab;
+      lay_out_class(L, t.out, false);
+      if (int rc = clear_ket_pads(t.out, s)) return rc;
+      t.elem0 = elems;
+      elems += (int64_t)t.Kab * t.npairs;
+      meta.push_back(t);
     }
-    LAI_CUDA_TRY(cudaMemcpyAsync(d_meta.p, v.data(), sizeof(ClassTables) * nc, cudaMemcpyHostToDevice, s));
-    build_tables_kernel<<<blocks_for(nelem), 256, 0, s>>>(d_meta.as<ClassTables>(), nc, nelem, dp, nullptr, nullptr,
-                                                          nullptr, ds, de, dcf);
+    LAI_CUDA_TRY(cudaMemcpyAsync(d_meta.p, meta.data(), sizeof(ClassTables) * meta.size(), cudaMemcpyHostToDevice, s));
+    build_tables_kernel<<<blocks_for(elems), 256, 0, s>>>(d_meta.as<ClassTables>(), (int)meta.size(), elems, dp,
+                                                          nullptr, nullptr, nullptr, ds, de, dcf);
     LAI_CUDA_TRY(cudaGetLastError());
     LaunchLanes lanes(E, s, kLanes);
-    for (int c = nc - 1; c >= 0; --c) {
-      if (v[c].npairs == 0) continue;
+    for (size_t i = first; i < last; ++i) {
+      const Piece& pc = pieces[i];
+      const auto& o = pc.tab.out;
       lai::QuartetBlock blk{};
-      blk.bra = blk.ket = v[c].out;
+      blk.bra = blk.ket = o;
       blk.offsets = iota64;
       blk.qbegin = iota32;
-      blk.total = v[c].npairs;
+      blk.total = o.npairs;
       blk.same_class = 1;
       lai::JKArgs args{};
       args.mode = lai::MODE_SCHWARZ;
-      args.schwarz_out = stage == 0 ? d_q + raw[c].pair0 : d_qprim + raw[c].elem0;
-      const auto& o = v[c].out;
-      cudaError_t ce = lanes.pick(alg_work(o.la, o.lb, o.la, o.lb, o.Ka, o.Kb, o.Ka, o.Kb) * v[c].npairs, &E->stream);
+      args.schwarz_out = pc.stage == 0 ? d_q + pc.pair0 : d_qprim + pc.prim0;
+      cudaError_t ce = lanes.pick(alg_work(o.la, o.lb, o.la, o.lb, o.Ka, o.Kb, o.Ka, o.Kb) * o.npairs, &E->stream);
       const int rc = ce == cudaSuccess ? launch_block(E, blk, args) : fail(LAI_ECUDA, cudaGetErrorString(ce));
       E->stream = s;
       if (rc) return rc;
@@ -363,6 +411,7 @@ int setup_pairs(lai_engine* E) {
   std::vector<double> Q(npairs);
   LAI_CUDA_TRY(cudaMemcpyAsync(Q.data(), d_q, sizeof(double) * npairs, cudaMemcpyDeviceToHost, s));
   LAI_CUDA_TRY(cudaStreamSynchronize(s));
+  LAI_CUDA_TRY(d_tmp.alloc(0));  // given back before the engine's own tables are taken
 
   // ---- screening and order (host) ----
   double qmax = 0.0;
