@@ -333,10 +333,9 @@ int upload_class(PairClassHost& c) {
 }
 
 int ensure_scratch(lai_engine* E, size_t doubles) {
-  if (doubles <= E->scratch_doubles) return LAI_OK;
+  if (E->d_scratch.bytes >= doubles * sizeof(double)) return LAI_OK;
   E->release_graph();
   LAI_CUDA_TRY(E->d_scratch.alloc(doubles * sizeof(double)));
-  E->scratch_doubles = doubles;
   return LAI_OK;
 }
 
@@ -512,7 +511,7 @@ int launch_block(lai_engine* E, const lai::QuartetBlock& blk, const lai::JKArgs&
   if (int rc = ensure_scratch(E, need)) return rc;
   // one scratch buffer: launches that use it follow one another on the caller's stream
   const int rc = lai::launch_generic(blk, args, E->tab, E->fork_stream ? E->fork_stream : E->stream,
-                                     E->d_scratch.as<double>(), E->scratch_doubles, E->num_sms);
+                                     E->d_scratch.as<double>(), E->d_scratch.bytes / sizeof(double), E->num_sms);
   if (rc < 0) return fail(LAI_ECUDA, std::string("generic launch failed: ") +
                                          cudaGetErrorString(cudaGetLastError()));
   return LAI_OK;
@@ -541,7 +540,7 @@ __global__ void absmax_kernel(const double* __restrict__ x, size_t n, unsigned l
 
 // max |x_i| of a device array (one stream synchronisation).
 int device_absmax(lai_engine* E, const double* x, size_t n, cudaStream_t stream, double* out) {
-  if (E->d_absmax.bytes < sizeof(unsigned long long)) LAI_CUDA_TRY(E->d_absmax.alloc(sizeof(unsigned long long)));
+  LAI_CUDA_TRY(E->d_absmax.ensure(sizeof(unsigned long long)));
   LAI_CUDA_TRY(cudaMemsetAsync(E->d_absmax.p, 0, sizeof(unsigned long long), stream));
   if (n > 0) {
     const size_t want = (n + 255) / 256;
@@ -790,9 +789,7 @@ int enqueue_jk(lai_engine* E, const double* dD, cudaStream_t stream, const lai_j
     }
     E->prof_block.clear();
     E->prof_quartets.clear();
-    if (E->d_prof_prims.bytes < sizeof(unsigned long long) * nparts * E->blocks.size())
-      LAI_CUDA_TRY(E->d_prof_prims.alloc(sizeof(unsigned long long) *
-                                         std::max<size_t>(1, nparts * E->blocks.size())));
+    LAI_CUDA_TRY(E->d_prof_prims.ensure(sizeof(unsigned long long) * std::max<size_t>(1, nparts * E->blocks.size())));
     LAI_CUDA_TRY(cudaMemsetAsync(E->d_prof_prims.p, 0, E->d_prof_prims.bytes, stream));
   }
   E->prof_n = 0;
@@ -1262,11 +1259,7 @@ int lai_jk_build(lai_engine* engine, const double* D, size_t nbf, double* J, dou
   }
   LAI_CUDA_TRY(cudaSetDevice(engine->device));
   const size_t bytes = sizeof(double) * nbf * nbf;
-  if (engine->d_D.bytes < bytes) {
-    LAI_CUDA_TRY(engine->d_D.alloc(bytes));
-    LAI_CUDA_TRY(engine->d_J.alloc(bytes));
-    LAI_CUDA_TRY(engine->d_K.alloc(bytes));
-  }
+  for (DevBuf* b : {&engine->d_D, &engine->d_J, &engine->d_K}) LAI_CUDA_TRY(b->ensure(bytes));
   cudaStream_t s = engine->stream;
   LAI_CUDA_TRY(cudaMemcpyAsync(engine->d_D.p, D, bytes, cudaMemcpyHostToDevice, s));
   if (int rc = run_jk(engine, engine->d_D.as<double>(), engine->d_J.as<double>(),
@@ -1297,11 +1290,7 @@ int lai_jk_build_batched(lai_engine* engine, const double* D, double* J, double*
     return fail(LAI_EINVAL, "lai_jk_build_batched: fp32_prim_rel must be in [0, 1)");
   LAI_CUDA_TRY(cudaSetDevice(engine->device));
   const size_t bytes = sizeof(double) * engine_mat_elems(engine);
-  if (engine->d_D.bytes < bytes) {
-    LAI_CUDA_TRY(engine->d_D.alloc(bytes));
-    LAI_CUDA_TRY(engine->d_J.alloc(bytes));
-    LAI_CUDA_TRY(engine->d_K.alloc(bytes));
-  }
+  for (DevBuf* b : {&engine->d_D, &engine->d_J, &engine->d_K}) LAI_CUDA_TRY(b->ensure(bytes));
   cudaStream_t s = engine->stream;
   LAI_CUDA_TRY(cudaMemcpyAsync(engine->d_D.p, D, bytes, cudaMemcpyHostToDevice, s));
   if (int rc = run_jk(engine, engine->d_D.as<double>(), engine->d_J.as<double>(), engine->d_K.as<double>(), s, o,

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/libaccint_b200.h"
+#include "dev_buf.h"
 #include "eri_device.cuh"
 #include "eri_kernels.h"
 
@@ -28,22 +29,6 @@ int fail(int code, const std::string& msg);
       return fail(e_ == cudaErrorMemoryAllocation ? LAI_ENOMEM : LAI_ECUDA,             \
                   std::string(#expr) + ": " + cudaGetErrorString(e_));                  \
   } while (0)
-
-struct DevBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  DevBuf() = default;
-  DevBuf(const DevBuf&) = delete;
-  DevBuf& operator=(const DevBuf&) = delete;
-  ~DevBuf() { if (p) cudaFree(p); }
-  cudaError_t alloc(size_t n) {
-    if (p) { cudaFree(p); p = nullptr; }
-    bytes = n;
-    if (n == 0) return cudaSuccess;
-    return cudaMalloc(&p, n);
-  }
-  template <typename T> T* as() const { return static_cast<T*>(p); }
-};
 
 // Stream-ordered scratch of one call (cudaFreeAsync gives it back), from a memory pool of
 // this library that keeps up to 32 MB: the default pool returns its memory at every
@@ -179,8 +164,7 @@ struct lai_engine {
   lai::host::DevBuf d_JKp, d_D, d_J, d_K;
   double* jp() const { return d_JKp.as<double>(); }
   double* kp(size_t elems) const { return d_JKp.as<double>() + elems; }  // elems: all of J' (every accumulator)
-  lai::host::DevBuf d_scratch;
-  size_t scratch_doubles = 0;
+  lai::host::DevBuf d_scratch;    // of the generic kernel
   lai::host::DevBuf d_status;
   double split_cut = -1.0;       // FP32 cut the blocks' mixed-precision split was built for
   lai::host::DevBuf d_absmax;
@@ -190,7 +174,6 @@ struct lai_engine {
   // (la, lb) class (built on first use; one_electron.cu)
   lai::host::DevBuf d_1e_shell, d_1e_exp, d_1e_coef, d_1e_pairs, d_1e_charges;
   std::vector<int> one_e_class;    // per class: la, lb, first pair, pair count
-  size_t charges_cap = 0;
   // CUDA graph of one device build (lai_jk_opts.graph) and what it was captured for
   struct GraphKey {
     const double* D;

@@ -102,10 +102,9 @@ int lai_one_electron_device(lai_engine* engine, int op, int ncharge, const doubl
       ch[4 * c + 2] = charge_xyz[3 * c + 2];
       ch[4 * c + 3] = charge_q[c];
     }
-    if ((size_t)nc > engine->charges_cap) {
+    if (engine->d_1e_charges.bytes < sizeof(double) * ch.size()) {
       LAI_CUDA_TRY(cudaStreamSynchronize(s));
       LAI_CUDA_TRY(engine->d_1e_charges.alloc(sizeof(double) * ch.size()));
-      engine->charges_cap = nc;
     }
     LAI_CUDA_TRY(cudaMemcpyAsync(engine->d_1e_charges.p, ch.data(), sizeof(double) * ch.size(),
                                  cudaMemcpyHostToDevice, s));
