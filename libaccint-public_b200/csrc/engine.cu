@@ -423,12 +423,29 @@ void release_lanes(LaneSet& set) {
   set = LaneSet{};
 }
 
+// Id of the capture that the stream is part of, 0 if none.
+static unsigned long long capture_of(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) return 0;
+  return status == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
 LaunchLanes::LaunchLanes(lai_engine* E, cudaStream_t stream, size_t lanes) : E_(E), main_(stream), load_(1, 0.0), lock_(E->lanes_mutex) {
   E->fork_stream = stream;
   lanes = std::min(lanes, E->lanes.side.size() + 1);
   if (lanes < 2) return;
-  if (cudaEventRecord(E->lanes.ev[0], stream) != cudaSuccess) return;  // one lane: the caller's stream
+  // A side stream of an earlier call inside a capture belongs to that capture until it
+  // ends, and another stream's work may not be queued on it.
+  const unsigned long long own = capture_of(stream);
   load_.resize(lanes, -1.0);
+  bool any = false;
+  for (size_t i = 1; i < lanes; ++i) {
+    const unsigned long long c = capture_of(E->lanes.side[i - 1]);
+    if (c && c != own) load_[i] = kClosed;
+    else any = true;
+  }
+  if (!any || cudaEventRecord(E->lanes.ev[0], stream) != cudaSuccess) load_.resize(1);  // one lane: the caller's stream
 }
 
 cudaError_t LaunchLanes::pick(double work, cudaStream_t* s) {
@@ -447,7 +464,7 @@ cudaError_t LaunchLanes::pick(double work, cudaStream_t* s) {
 cudaError_t LaunchLanes::join() {
   cudaError_t rc = cudaSuccess;
   for (size_t i = 1; i < load_.size(); ++i) {
-    if (load_[i] < 0.0) continue;
+    if (load_[i] < 0.0 || load_[i] == kClosed) continue;
     cudaError_t e = cudaEventRecord(E_->lanes.ev[i], E_->lanes.side[i - 1]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(main_, E_->lanes.ev[i], 0);
     if (e != cudaSuccess) rc = e;

@@ -264,9 +264,11 @@ class LaunchLanes {
  private:
   lai_engine* E_;
   cudaStream_t main_;
+  static constexpr double kClosed = 1e300;
   std::vector<double> load_;   // estimated work per lane; < 0: not forked yet
-  // calls of several threads on one engine queue their launches one after another (they
-  // share the lanes' events)
+  // Gradients and density-fitting integrals of several threads on one engine queue their
+  // launches one after another: they share the lanes' events.  (J/K builds share the
+  // accumulators as well, and are the caller's to serialize.)
   std::unique_lock<std::mutex> lock_;
 };
 double alg_work(int la, int lb, int lc, int ld, int Ka, int Kb, int Kc, int Kd);

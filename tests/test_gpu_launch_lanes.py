@@ -60,3 +60,39 @@ def test_engines_of_several_threads_share_the_pool():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("call", ["jk"])
+def test_calls_beside_a_capture_that_is_still_open(call):
+    """Between a captured call and the end of its capture, the engine's side streams are the
+    capture's: a call on another stream runs beside it, and the capture stays good."""
+    import torch
+    w = lai.workloads.make("h2o2_631g")
+    eng = lai.Engine(w.basis)
+    J0, K0, _ = eng.jk(w.D)
+    g0 = eng.gradient(w.D)
+    d = torch.from_numpy(w.D).cuda()
+    out = [[torch.empty_like(d) for _ in range(2)] for _ in range(2)]
+    grad = [torch.empty(eng.natom(), 3, dtype=torch.float64, device="cuda") for _ in range(2)]
+
+    def run(k, stream):
+        if call == "jk":
+            eng.jk_device(d.data_ptr(), out[k][0].data_ptr(), out[k][1].data_ptr(), stream=stream.cuda_stream)
+        else:
+            lai._lib.check(lai._lib.lib().lai_jk_gradient_device(eng._h, d.data_ptr(), grad[k].data_ptr(),
+                                                                 stream.cuda_stream))
+
+    graph, inside, beside = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=inside, capture_error_mode="thread_local"):
+        run(0, inside)
+        run(1, beside)
+    beside.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    for k in range(2):
+        if call == "jk":
+            for a, b in zip(out[k], (J0, K0)):
+                assert np.max(np.abs(a.cpu().numpy() - b)) < REL * np.max(np.abs(b))
+        else:
+            assert np.max(np.abs(grad[k].cpu().numpy() - g0)) < 1e-12 * np.max(np.abs(g0))
