@@ -170,6 +170,9 @@ struct lai_engine {
   lai::host::DevBuf d_absmax;
   lai::host::DevBuf d_shell_atom;  // [nshell] atom of each shell (gradients)
   int natom = -1;
+  lai::host::DevBuf d_grad_acc;    // accumulators of a gradient, after grad_done
+  cudaEvent_t grad_done = nullptr;
+  std::mutex grad_mutex;
   // one-electron integrals: shell table, primitives and shell pairs grouped by
   // (la, lb) class (built on first use; one_electron.cu)
   lai::host::DevBuf d_1e_shell, d_1e_exp, d_1e_coef, d_1e_pairs, d_1e_charges;
@@ -226,6 +229,7 @@ struct lai_engine {
 inline lai_engine::~lai_engine() {
   release_graph();
   for (auto e : prof_ev) cudaEventDestroy(e);
+  if (grad_done) cudaEventDestroy(grad_done);
   classes.clear();
   blocks.clear();
   lai::host::release_lanes(lanes);

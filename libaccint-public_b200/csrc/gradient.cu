@@ -39,11 +39,35 @@ __global__ void sum_copies_kernel(const double* __restrict__ copies, int stride,
   grad[i] = s;
 }
 
-// Stream-ordered scratch of one call (calls of several threads or streams do not share it).
-struct StreamBuf {
+// The accumulators of one call.  A call outside a capture uses the engine's, after the work
+// of the call before it, whatever stream that went to: an allocation per call, also from a
+// pool, is refused in a thread that is capturing, and breaks a global capture of another
+// thread.  Inside a capture they are the graph's own.
+struct Accumulators {
+  lai_engine* E;
+  cudaStream_t s;
+  std::unique_lock<std::mutex> lock;  // until the call's work is queued
   void* p = nullptr;
-  cudaStream_t s = nullptr;
-  ~StreamBuf() { if (p) cudaFreeAsync(p, s); }
+  bool owned = false;
+  Accumulators(lai_engine* engine, cudaStream_t stream) : E(engine), s(stream), lock(engine->grad_mutex) {}
+  int take(size_t bytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    LAI_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+      LAI_CUDA_TRY(scratch_alloc(&p, bytes, s));
+      owned = true;
+      return LAI_OK;
+    }
+    if (!E->grad_done) LAI_CUDA_TRY(cudaEventCreateWithFlags(&E->grad_done, cudaEventDisableTiming));
+    LAI_CUDA_TRY(E->d_grad_acc.ensure(bytes));
+    LAI_CUDA_TRY(cudaStreamWaitEvent(s, E->grad_done, 0));
+    p = E->d_grad_acc.p;
+    return LAI_OK;
+  }
+  ~Accumulators() {
+    if (owned) cudaFreeAsync(p, s);
+    else if (p) cudaEventRecord(E->grad_done, s);
+  }
 };
 
 }  // namespace
@@ -65,9 +89,8 @@ int lai_jk_gradient_device(lai_engine* engine, const double* d_D, double* d_grad
   cudaStream_t stream_of_call = static_cast<cudaStream_t>(stream);
   const int n3 = 3 * engine->natom, stride = (n3 + 15) / 16 * 16;
   const size_t bytes = sizeof(double) * stride * lai::kGradCopies;
-  StreamBuf copies;
-  copies.s = stream_of_call;
-  LAI_CUDA_TRY(scratch_alloc(&copies.p, bytes, stream_of_call));
+  Accumulators copies(engine, stream_of_call);
+  if (int rc = copies.take(bytes)) return rc;
   double* const acc = static_cast<double*>(copies.p);
   LAI_CUDA_TRY(cudaMemsetAsync(acc, 0, bytes, stream_of_call));
   const int nbf = (int)engine->basis->nbf;

@@ -62,7 +62,7 @@ def test_engines_of_several_threads_share_the_pool():
     assert not bad
 
 
-@pytest.mark.parametrize("call", ["jk"])
+@pytest.mark.parametrize("call", ["jk", "gradient"])
 def test_calls_beside_a_capture_that_is_still_open(call):
     """Between a captured call and the end of its capture, the engine's side streams are the
     capture's: a call on another stream runs beside it, and the capture stays good."""
