@@ -7,11 +7,15 @@
 
 namespace lai {
 
+// FP64: from ld = 2 on the f shells start at 0 (expansion about M, eri_block_impl.cuh)
 #define LAI_BLOCK_KETS(K)                                                                              \
-  K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 2, 4) K(3, 0, 3, 3)     \
-  K(3, 1, 3, 4) K(3, 2, 3, 5) K(3, 3, 3, 6) K(4, 0, 4, 4) K(4, 1, 4, 5) K(4, 2, 4, 6)                  \
+  K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 0, 4) K(3, 0, 3, 3)     \
+  K(3, 1, 3, 4) K(3, 2, 0, 5) K(3, 3, 0, 6) K(4, 0, 4, 4) K(4, 1, 4, 5) K(4, 2, 0, 6)                  \
   /* more components than a thread's registers hold: two launches, each digests its part */           \
-  K(4, 3, 4, 5) K(4, 3, 6, 7) K(4, 4, 4, 6) K(4, 4, 7, 8)
+  K(4, 3, 0, 5) K(4, 3, 6, 7) K(4, 4, 0, 6) K(4, 4, 7, 8)
+#define LAI_BLOCK_KETS_F32(K)                                                                          \
+  K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 2, 4) K(3, 0, 3, 3)     \
+  K(3, 1, 3, 4) K(3, 2, 3, 5) K(3, 3, 3, 6)
 
 namespace block_detail {
 #define K(c, d, f0, f1)                                                                                       \
@@ -24,8 +28,7 @@ LAI_BLOCK_KETS(K)
 #define K(c, d, f0, f1) \
   extern template int launch_range<c, d, f0, f1, float>(const QuartetBlock&, const JKArgs&, const RysTablesView&, \
                                                         cudaStream_t, int);
-K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 2, 4) K(3, 0, 3, 3) K(3, 1, 3, 4)
-K(3, 2, 3, 5) K(3, 3, 3, 6)
+LAI_BLOCK_KETS_F32(K)
 #undef K
 }  // namespace block_detail
 
@@ -45,12 +48,15 @@ int launch_blockq(const QuartetBlock& blk, const JKArgs& args, const RysTablesVi
   if (args.mode != MODE_JK) return -1;
   if (blk.total - blk.t_begin <= 0) return 0;
   const int lc = blk.ket.la, ld = blk.ket.lb;
-#define K(c, d, f0, f1)                                                                               \
-  if (lc == c && ld == d) {                                                                           \
-    if constexpr (c < 4)                                                                              \
-      if (fp32) return block_detail::launch_range<c, d, f0, f1, float>(blk, args, tab, stream, num_sms); \
-    if (const int rc = block_detail::launch_range<c, d, f0, f1, double>(blk, args, tab, stream, num_sms)) return rc; \
+  if (fp32) {
+#define K(c, d, f0, f1) \
+  if (lc == c && ld == d) return block_detail::launch_range<c, d, f0, f1, float>(blk, args, tab, stream, num_sms);
+    LAI_BLOCK_KETS_F32(K)
+#undef K
   }
+#define K(c, d, f0, f1)                                                                               \
+  if (lc == c && ld == d)                                                                             \
+    if (const int rc = block_detail::launch_range<c, d, f0, f1, double>(blk, args, tab, stream, num_sms)) return rc;
   LAI_BLOCK_KETS(K)
 #undef K
   return 0;

@@ -22,6 +22,20 @@
 //      F0..F1 of f.
 // The density blocks arrive by cp.async behind the table phase.
 //
+// Expansion centre.  The transfer writes (x-A)^a (x-B)^b in powers of x-A, and where A lies
+// far from the charge the terms are large and cancel: on one side by up to some ten times, on
+// both sides by the product.  Applied per root to the 2-D tables, as the tiled kernel does,
+// it costs the sum over directions; applied to the contracted block the product over
+// directions and sides: K' of (ff|ff) in H2O/cc-pVQZ was off by 4.8e-14 of its norm where the
+// tiled kernel is off by 2.1e-15.  So a ket with ld >= 2, and a bra with la >= 3 and lb >= 2
+// against a ket with ld >= 1 (from lb = 3 also (ds|, (fs| and (gs| kets; template parameter
+// BM), are expanded about M, the centre P of the pair's first primitive: powers 0..la+lb of
+// x-M, (x-A)^a = (x-M + M-A)^a and the same for B, whose terms are as large as the charge
+// makes them.  K' of (ff|ff): 1.5e-15; J and K of H2O/cc-pVQZ, in three geometries, 7e-15 to
+// 1e-14 before and 4e-15 now.  The other classes are as exact as the tiled kernel without it.
+// It costs rows ((fd| 56 for 46) and longer bra sums (prod (a_x + b_x + 1) terms for
+// prod (b_x + 1)): (fd|dp) of C6H14/cc-pVTZ 2.37 -> 2.72 ms, the build 84.2 -> 86.1 ms.
+//
 // R = double, or float for the FP32 part of a mixed-precision build (roots, tables and the
 // primitive sums in G in FP32; the primitive-pair quantities up to T and the prefactor,
 // and everything after G, in FP64).
@@ -60,7 +74,8 @@ __host__ __device__ constexpr int odd_stride(int n) {
   return u * (((n + u - 1) / u) | 1);
 }
 
-constexpr int kMaxThreads = 160;  // components of (gg|: 145
+constexpr int kMaxThreads = 160;     // components of (gg| about A: 145
+constexpr int kMaxThreadsMid = 192;  // and about M: 165
 constexpr int kMaxTerms = 12;     // transfer terms of a g component: (2,1,1) -> 3 * 2 * 2
 constexpr int kMaxLab = 2 * kMaxL;
 constexpr int kMaxSmem = 226 * 1024;  // of 227 KB, less the static part
@@ -72,10 +87,10 @@ constexpr int kMaxSmem = 226 * 1024;  // of 227 KB, less the static part
 // with them: (fd|ps) 4.9 -> 3.5 ms, (ff|ps) 1.6 -> 0.9, (fs|dp) 4.8 -> 4.0, (fd|pp) 1.75 ->
 // 1.67, but (dd|pp) 2.5 -> 2.8; from 25 components on the spills cost more ((dd|fp) 1.2 ->
 // 1.6 with 128).
-template <int F0, int F1>
-__host__ __device__ constexpr int min_blocks() {
+template <int F0, int F1, bool BM>
+__host__ __device__ constexpr int min_blocks() {  // (BM: blocks of 192 threads, nearly the same caps)
   constexpr int nf = ncart_range(F0, F1);
-  return nf <= 10 ? 4 : nf <= 16 ? 3 : 1;
+  return nf <= 10 ? 4 - BM : nf <= 16 ? 3 - BM : 1;
 }
 
 __host__ __device__ constexpr int block_binom(int n, int k) {
@@ -87,6 +102,31 @@ __device__ __forceinline__ double block_pow(double x, int m) {
   double r = 1.0;
   for (int i = 0; i < m; ++i) r *= x;
   return r;
+}
+
+// Expansion about M instead of the first shell's centre (see above).
+template <int LD, typename R>
+__host__ __device__ constexpr bool mid_ket() { return sizeof(R) == 8 && LD >= 2; }
+template <int LC, int LD, typename R>
+__host__ __device__ constexpr bool mid_bra_possible() { return sizeof(R) == 8 && (LD >= 1 || LC >= 2); }
+__host__ __device__ constexpr bool mid_bra(int la, int lb, int ld) { return la >= 3 && lb >= (ld > 0 ? 2 : 3); }
+
+// out[k] = coefficient of x^k in (x + p)^i (x + q)^j, k <= i + j < N.
+template <int N>
+__device__ __forceinline__ void mid_coefs(double p, double q, int i, int j, double* out) {
+  double c[N];
+  c[0] = 1.0;
+#pragma unroll
+  for (int k = 1; k < N; ++k) c[k] = 0.0;
+  for (int m = 0; m < i + j; ++m) {
+    const double r = m < i ? p : q;
+#pragma unroll
+    for (int k = N - 1; k > 0; --k) c[k] = c[k - 1] + r * c[k];
+    c[0] *= r;
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (k <= i + j) out[k] = c[k];
 }
 
 // Ket components c per digestion chunk (a divisor of the shell's count): enough values
@@ -109,7 +149,7 @@ struct BlockGeom {
   int doubles;   // total, including the integer tables at o_int
 };
 
-template <int LC, int LD, typename R>
+template <int LC, int LD, typename R, bool BM>
 __host__ BlockGeom make_geom(int la, int lb, int threads, int batch) {
   constexpr int W = LC + LD + 1, WS = odd_stride<R>(W), ND = ncart(LD), NC = ncart(LC);
   constexpr int CB = chunk_components(LC, LD), NV = CB * ND, NVP = odd_stride(NV);
@@ -117,7 +157,7 @@ __host__ BlockGeom make_geom(int la, int lb, int threads, int batch) {
   BlockGeom g{};
   g.la = la; g.lb = lb;
   g.nroots = (la + lb + LC + LD) / 2 + 1;
-  g.ne = ncart_range(la, la + lb);
+  g.ne = ncart_range(BM ? 0 : la, la + lb);
   g.na = ncart(la); g.nb = ncart(lb); g.nab = g.na * g.nb;
   g.nacc = g.nab + NC * ND + g.na * NC + g.na * ND + g.nb * NC + g.nb * ND;
   g.batch = batch;
@@ -134,15 +174,16 @@ __host__ BlockGeom make_geom(int la, int lb, int threads, int batch) {
   g.o_jab = take(g.nab);
   g.o_kad = take(g.na * ND + g.nb * ND);
   g.o_kbd = g.o_kad + g.na * ND;
-  g.o_cob = take(g.nb * kMaxTerms);
-  g.o_cod = take(ND * kMaxTerms);
+  g.o_cob = take(BM ? 3 * (la + 1) * (lb + 1) * (la + lb + 1) : g.nb * kMaxTerms);
+  g.o_cod = take(mid_ket<LD, R>() ? 3 * (LC + 1) * (LD + 1) * W : ND * kMaxTerms);
   g.o_nab = take(g.nab);
   g.o_ncd = take(NC * ND);
   g.o_int = o;
-  // integers: list of primitive quartets (64-bit), (e0| index of every bra term, per-b
-  // term count, coefficient and powers, the same coefficients and powers for the ket, row
-  // and column of every density element
-  const int ints = 2 * threads + g.nab * kMaxTerms + g.nb * (1 + 2 * kMaxTerms) + ND * 2 * kMaxTerms + g.nacc + 8;
+  // integers: list of primitive quartets (64-bit), (e0| index of every bra term (BM: of every
+  // power of x, y and z), per-b term count, coefficient and powers, the same coefficients
+  // and powers for the ket, row and column of every density element
+  const int terms = BM ? (la + lb + 1) * (la + lb + 1) * (la + lb + 1) : g.nab * kMaxTerms;
+  const int ints = 2 * threads + terms + g.nb * (1 + 2 * kMaxTerms) + ND * 2 * kMaxTerms + g.nacc + 8;
   o += (ints + 1) / 2;
   g.doubles = (o + 1) & ~1;
   return g;
@@ -171,14 +212,15 @@ __device__ __forceinline__ int find_bra_warp(const int64_t* __restrict__ offsets
   return lo;
 }
 
-template <int LC, int LD, int F0, int F1, typename R>
-__global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
+template <int LC, int LD, int F0, int F1, typename R, bool BM>
+__global__ void __launch_bounds__((BM ? kMaxThreadsMid : kMaxThreads), (min_blocks<F0, F1, BM>()))
     eri_block_kernel(QuartetBlock one, JKArgs args, RysTablesView tab, BlockGeom g, int nsplit1, int csplit1,
                      const MultiEntry* list_of_blocks, int nblocks, int64_t nwork) {
   constexpr int LCD = LC + LD, W = LCD + 1, WS = odd_stride<R>(W);
   constexpr int NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
   constexpr int CB = chunk_components(LC, LD), NV = CB * ND, NVP = odd_stride(NV);
   constexpr int NF = ncart_range(F0, F1);
+  constexpr bool KM = mid_ket<LD, R>();
   extern __shared__ __align__(16) double smem_b[];
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
   const int la = g.la, lb = g.lb, LAB = la + lb, NR = g.nroots;
@@ -197,13 +239,14 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
   double* const Dbd = Dbc + NB * NC;
   double* const Jab = smem_b + g.o_jab;
   double* const Kxd = smem_b + g.o_kad;   // K'_ad, then K'_bd
-  double* const CoB = smem_b + g.o_cob;   // per quartet: coefficient of bra term (b, t)
-  double* const CoD = smem_b + g.o_cod;   // per quartet: coefficient of ket term (d, t)
+  double* const CoB = smem_b + g.o_cob;   // per quartet: coefficient of bra term (b, t), or (BM) of
+                                          // x^k in (x+M-A)^i (x+M-B)^j by direction, i, j and k
+  double* const CoD = smem_b + g.o_cod;   // the same for the ket: term (d, t), or (KM) direction, i, j, k
   double* const Nab = smem_b + g.o_nab;   // normalization of (a, b)
   double* const Ncd = smem_b + g.o_ncd;
   int64_t* const list = reinterpret_cast<int64_t*>(smem_b + g.o_int);
   int* const be = reinterpret_cast<int*>(list + nt);  // [ab][term] index of a + k
-  int* const bn = be + NAB * kMaxTerms;
+  int* const bn = be + (BM ? (LAB + 1) * (LAB + 1) * (LAB + 1) : NAB * kMaxTerms);
   int* const bc = bn + NB;
   int* const bp = bc + NB * kMaxTerms;
   int* const dc = bp + NB * kMaxTerms;
@@ -212,8 +255,16 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
   int* const nlist = dpos + g.nacc;
 
   // ---- tables of the class, once per block ----
+  if constexpr (BM)
+    for (int i = tid; i < (LAB + 1) * (LAB + 1) * (LAB + 1); i += nt) {
+      const int x = i / ((LAB + 1) * (LAB + 1)), yz = i - x * (LAB + 1) * (LAB + 1);
+      const int y = yz / (LAB + 1), z = yz - y * (LAB + 1);
+      be[i] = x + y + z <= LAB ? ncart_before(0, x + y + z) + cart_index(x, y, z) : 0;
+    }
   for (int i = tid; i < NAB; i += nt) {
     const int a = i / NB, b = i - a * NB;
+    Nab[i] = norm_factor(la, a) * norm_factor(lb, b);
+    if constexpr (BM) continue;
     const int ca = cart_comp(la, a), cb = cart_comp(lb, b);
     const int bx = comp_x(cb), by = comp_y(cb), bz = comp_z(cb);
     int t = 0;
@@ -228,11 +279,10 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
           }
         }
     if (a == 0) bn[b] = t;
-    Nab[i] = norm_factor(la, a) * norm_factor(lb, b);
   }
   for (int i = tid; i < NCD; i += nt) {
     Ncd[i] = norm_factor(LC, i / ND) * norm_factor(LD, i % ND);
-    if (i < ND) {
+    if (!KM && i < ND) {
       const int cd = cart_comp(LD, i);
       const int dx = comp_x(cd), dy = comp_y(cd), dz = comp_z(cd);
       int t = 0;
@@ -259,7 +309,7 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
   // this thread's rows of the tables
   int ox = 0, oy = g.ts, oz = 2 * g.ts;
   if (tid < NE) {
-    int l = la, r = tid;
+    int l = BM ? 0 : la, r = tid;
     while (r >= ncart(l)) r -= ncart(l++);
     const int ce = cart_comp(l, r);
     ox += comp_x(ce) * WS;
@@ -316,6 +366,10 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
       const double sym = quartet_weight(blk, p, q);
       const SysMats mats = sys_mats(args, blk, p);
       const size_t n = (size_t)mats.nbf;
+      const double* __restrict__ pbra = blk.bra.primb + (size_t)p * Kab * kBraRec;
+      const double* __restrict__ pket = blk.ket.primb + (size_t)q * Kcd * kBraRec;
+      const bool one_centre = BM && __ldg(blk.bra.AB + p) == 0.0 && __ldg(blk.bra.AB + nbra + p) == 0.0 &&
+                              __ldg(blk.bra.AB + 2 * nbra + p) == 0.0;
       {  // density blocks, transfer coefficients, zeroed sums
         const double* __restrict__ D = mats.D;
         auto first = [&](int sh) { return sh == 0 ? fa : sh == 1 ? fb : sh == 2 ? fc : fd; };
@@ -327,13 +381,31 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
         for (int i = tid; i < (NA + NB) * ND; i += nt) Kxd[i] = 0.0;
         const double ABx = __ldg(blk.bra.AB + p), ABy = __ldg(blk.bra.AB + nbra + p),
                      ABz = __ldg(blk.bra.AB + 2 * nbra + p);
-        for (int i = tid; i < NB * kMaxTerms; i += nt) {
-          if (i % kMaxTerms >= bn[i / kMaxTerms]) continue;
-          const int k = bp[i];
-          CoB[i] = (double)bc[i] * block_pow(ABx, k & 15) * block_pow(ABy, (k >> 4) & 15) * block_pow(ABz, k >> 8);
+        if constexpr (BM) {
+          const int per = (la + 1) * (lb + 1);
+          for (int i = tid; i < 3 * per; i += nt) {
+            const int x = i / per, ij = i - x * per, ia = ij / (lb + 1);
+            const double pa = __ldg(pbra + BR_PAX + x);
+            mid_coefs<kMaxLab + 1>(pa, pa + (x == 0 ? ABx : x == 1 ? ABy : ABz), ia, ij - ia * (lb + 1),
+                                   CoB + i * (LAB + 1));
+          }
+        } else {
+          for (int i = tid; i < NB * kMaxTerms; i += nt) {
+            if (i % kMaxTerms >= bn[i / kMaxTerms]) continue;
+            const int k = bp[i];
+            CoB[i] = (double)bc[i] * block_pow(ABx, k & 15) * block_pow(ABy, (k >> 4) & 15) * block_pow(ABz, k >> 8);
+          }
         }
         const double CDx = __ldg(blk.ket.AB + q), CDy = __ldg(blk.ket.AB + nket + q),
                      CDz = __ldg(blk.ket.AB + 2 * nket + q);
+        if constexpr (KM) {
+          constexpr int per = (LC + 1) * (LD + 1);
+          for (int i = nt - 1 - tid; i < 3 * per; i += nt) {
+            const int x = i / per, ij = i - x * per, ic = ij / (LD + 1);
+            const double qc = __ldg(pket + BR_PAX + x);
+            mid_coefs<W>(qc, qc + (x == 0 ? CDx : x == 1 ? CDy : CDz), ic, ij - ic * (LD + 1), CoD + i * W);
+          }
+        } else
         for (int i = tid; i < ND * kMaxTerms; i += nt) {
           const int k = dp[i];
           CoD[i] = (double)dc[i] * block_pow(CDx, k & 15) * block_pow(CDy, (k >> 4) & 15) * block_pow(CDz, k >> 8);
@@ -345,8 +417,6 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
 
       // ---- primitive quartets: this block's candidates split + k * nsplit, those above
       // the cut collected in a list, the list processed `batch` at a time ----
-      const double* __restrict__ pbra = blk.bra.primb + (size_t)p * Kab * kBraRec;
-      const double* __restrict__ pket = blk.ket.primb + (size_t)q * Kcd * kBraRec;
       for (int64_t c0 = split; c0 < P; c0 += (int64_t)nt * nsplit) {
         int cnt;
         if (P == 1) {  // (the usual case of the d, f and g shells): no list
@@ -388,7 +458,10 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
             R u, w;
             rys_root_one<R>(NR, r, R(T), tab, u, w);
             const R pqx = R(x == 0 ? PQx : x == 1 ? PQy : PQz), rzr = R(rz), rer = R(re);
-            const R pa = R(__ldg(pb + BR_PAX + x)) - rzr * u * pqx, qc = R(__ldg(pk + BR_PAX + x)) + rer * u * pqx;
+            // P - A and Q - C, or P - M and Q - M (0 in the first primitive)
+            const double pc = BM ? __ldg(pb + BR_PX + x) - __ldg(pbra + BR_PX + x) : __ldg(pb + BR_PAX + x);
+            const double qd = KM ? __ldg(pk + BR_PX + x) - __ldg(pket + BR_PX + x) : __ldg(pk + BR_PAX + x);
+            const R pa = R(pc) - rzr * u * pqx, qc = R(qd) + rer * u * pqx;
             const R b00 = R(0.5) * R(inv) * u, b10 = R(hz) - R(hz) * rzr * u, b01 = R(he) - R(he) * rer * u;
             R* dst = Tb + (size_t)(s * NR * 3 + rx) * g.ts;
             R cur[kMaxLab + 1], prev[kMaxLab + 1];
@@ -476,6 +549,27 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
                 constexpr int i = decltype(II)::value;
                 constexpr int cc = cart_comp(LC, c0_ + i / ND), d = i % ND, cd = cart_comp(LD, d);
                 double h = 0.0;
+                if constexpr (KM) {
+                  constexpr int per = (LC + 1) * (LD + 1) * W;
+                  const double* cx = CoD + (comp_x(cc) * (LD + 1) + comp_x(cd)) * W;
+                  const double* cy = CoD + per + (comp_y(cc) * (LD + 1) + comp_y(cd)) * W;
+                  const double* cz = CoD + 2 * per + (comp_z(cc) * (LD + 1) + comp_z(cd)) * W;
+                  bfor<0, comp_x(cc) + comp_x(cd) + 1>([&](auto KX) {
+                    bfor<0, comp_y(cc) + comp_y(cd) + 1>([&](auto KY) {
+                      constexpr int kx = decltype(KX)::value, ky = decltype(KY)::value;
+                      constexpr int z0 = F0 - kx - ky > 0 ? F0 - kx - ky : 0;
+                      constexpr int z1 = comp_z(cc) + comp_z(cd) < F1 - kx - ky ? comp_z(cc) + comp_z(cd) : F1 - kx - ky;
+                      if constexpr (z0 <= z1) {
+                        double hz = 0.0;
+                        bfor<z0, z1 + 1>([&](auto KZ) {
+                          constexpr int kz = decltype(KZ)::value;
+                          hz += cz[kz] * G[ncart_before(F0, kx + ky + kz) + cart_index(kx, ky, kz)];
+                        });
+                        h += cx[kx] * cy[ky] * hz;
+                      }
+                    });
+                  });
+                } else
                 bfor<0, comp_x(cd) + 1>([&](auto KX) {
                   bfor<0, comp_y(cd) + 1>([&](auto KY) {
                     bfor<0, comp_z(cd) + 1>([&](auto KZ) {
@@ -502,16 +596,40 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
           double v[NVP];
 #pragma unroll
           for (int j = 0; j < NV; ++j) v[j] = 0.0;
-          const int terms = bn[b];
-          for (int k = 0; k < terms; ++k) {
-            const double co = CoB[b * kMaxTerms + k];
-            const double* h = Hs + be[i * kMaxTerms + k] * NVP;
+          auto add = [&](double co, int e) {
+            const double* h = Hs + e * NVP;
 #pragma unroll
             for (int j = 0; j < (NV + 1) / 2; ++j) {
               const double2 hv = *reinterpret_cast<const double2*>(h + 2 * j);
               v[2 * j] += co * hv.x;
               if (2 * j + 1 < NV) v[2 * j + 1] += co * hv.y;
             }
+          };
+          if constexpr (BM) {
+            const int ca = cart_comp(la, a), cb = cart_comp(lb, b), per = (la + 1) * (lb + 1) * (LAB + 1);
+            const int ax = comp_x(ca), ay = comp_y(ca), az = comp_z(ca);
+            const int bx = comp_x(cb), by = comp_y(cb), bz = comp_z(cb);
+            const double* cx = CoB + (ax * (lb + 1) + bx) * (LAB + 1);
+            const double* cy = CoB + per + (ay * (lb + 1) + by) * (LAB + 1);
+            const double* cz = CoB + 2 * per + (az * (lb + 1) + bz) * (LAB + 1);
+            // one loop over all powers, whose length is all that differs between the lanes (a
+            // pair on one centre has the highest powers only)
+            const int nx = ax + bx, ny = ay + by, nz = az + bz;
+            int kx = one_centre ? nx : 0, ky = one_centre ? ny : 0, kz = one_centre ? nz : 0;
+            const int terms = one_centre ? 1 : (nx + 1) * (ny + 1) * (nz + 1);
+            for (int k = 0; k < terms; ++k) {
+              add(cx[kx] * cy[ky] * cz[kz], be[(kx * (LAB + 1) + ky) * (LAB + 1) + kz]);
+              if (++kz > nz) {
+                kz = 0;
+                if (++ky > ny) {
+                  ky = 0;
+                  ++kx;
+                }
+              }
+            }
+          } else {
+            const int terms = bn[b];
+            for (int k = 0; k < terms; ++k) add(CoB[b * kMaxTerms + k], be[i * kMaxTerms + k]);
           }
           double sj = 0.0;
           const double nab = Nab[i];
@@ -581,21 +699,21 @@ __global__ void __launch_bounds__(kMaxThreads, (min_blocks<F0, F1>()))
       __syncthreads();  // before the next quartet's blocks overwrite these
     }
   }
-  if (F0 == LC) count_prims(args.prim_count, tid == 0 ? nprim_done : 0u);
+  if (F0 == (KM ? 0 : LC)) count_prims(args.prim_count, tid == 0 ? nprim_done : 0u);
 }
 
 // Geometry of a bra and its resident blocks per SM; -3 on a CUDA error.
-template <int LC, int LD, int F0, int F1, typename R>
+template <int LC, int LD, int F0, int F1, typename R, bool BM>
 int block_geometry(int la, int lb, int64_t P, BlockGeom* g, int* threads, size_t* smem) {
-  *threads = (ncart_range(la, la + lb) + 31) / 32 * 32;
+  *threads = (ncart_range(BM ? 0 : la, la + lb) + 31) / 32 * 32;
   const int nroots = (la + lb + LC + LD) / 2 + 1;
   // table batch: one thread per (primitive quartet, root, direction); a block of 32 has
   // room for at least one primitive quartet of its class (27 >= 3 nroots)
   int batch = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(P, 8), *threads / (3 * nroots)));
-  *g = make_geom<LC, LD, R>(la, lb, *threads, batch);
-  while (g->doubles * 8 > kMaxSmem && batch > 1) *g = make_geom<LC, LD, R>(la, lb, *threads, --batch);
+  *g = make_geom<LC, LD, R, BM>(la, lb, *threads, batch);
+  while (g->doubles * 8 > kMaxSmem && batch > 1) *g = make_geom<LC, LD, R, BM>(la, lb, *threads, --batch);
   *smem = sizeof(double) * (size_t)g->doubles;
-  auto kern = eri_block_kernel<LC, LD, F0, F1, R>;
+  auto kern = eri_block_kernel<LC, LD, F0, F1, R, BM>;
   // resident blocks per SM, per bra and batch (0: not asked yet)
   static std::atomic<int> occ[kMaxL + 1][kMaxL + 1][9];
   int per_sm = occ[la][lb][batch].load(std::memory_order_relaxed);
@@ -617,15 +735,14 @@ inline void block_split(int64_t nq, int64_t P, int batch, int nchunks, int64_t s
   *csplit = (int)std::max<int64_t>(1, std::min<int64_t>(nchunks, slots / (nq * *nsplit)));
 }
 
-// 0 when launched, -3 on a CUDA error.
-template <int LC, int LD, int F0, int F1, typename R>
-int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
-                 int num_sms) {
+template <int LC, int LD, int F0, int F1, typename R, bool BM>
+int launch_range_at(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
+                    int num_sms) {
   const int64_t P = (int64_t)blk.bra.Ka * blk.bra.Kb * blk.ket.Ka * blk.ket.Kb;
   BlockGeom g;
   int threads;
   size_t smem;
-  const int per_sm = block_geometry<LC, LD, F0, F1, R>(blk.bra.la, blk.bra.lb, P, &g, &threads, &smem);
+  const int per_sm = block_geometry<LC, LD, F0, F1, R, BM>(blk.bra.la, blk.bra.lb, P, &g, &threads, &smem);
   if (per_sm < 0) return per_sm;
   const int64_t nq = blk.total - blk.t_begin, slots = (int64_t)num_sms * per_sm;
   int nsplit, csplit;
@@ -635,9 +752,35 @@ int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesVie
   // least eight turns per block for balance
   g.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, nwork / (slots * 8)));
   const int64_t want = (nwork + g.chunk - 1) / g.chunk;
-  eri_block_kernel<LC, LD, F0, F1, R><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
+  eri_block_kernel<LC, LD, F0, F1, R, BM><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
       blk, args, tab, g, nsplit, csplit, nullptr, 0, nwork);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+template <int LC, int LD, int F0, int F1, bool BM>
+int launch_range_list_at(int la, int lb, int64_t Pmax, const MultiEntry* list, int n, int64_t nwork,
+                         const JKArgs& args, const RysTablesView& tab, cudaStream_t stream, int num_sms) {
+  BlockGeom g;
+  int threads;
+  size_t smem;
+  const int per_sm = block_geometry<LC, LD, F0, F1, double, BM>(la, lb, Pmax, &g, &threads, &smem);
+  if (per_sm < 0) return per_sm;
+  const int64_t slots = (int64_t)num_sms * per_sm;
+  g.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, nwork / (slots * 8)));
+  const int64_t want = (nwork + g.chunk - 1) / g.chunk;
+  eri_block_kernel<LC, LD, F0, F1, double, BM><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
+      QuartetBlock{}, args, tab, g, 1, 1, list, n, nwork);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// 0 when launched, -3 on a CUDA error.
+template <int LC, int LD, int F0, int F1, typename R>
+int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab, cudaStream_t stream,
+                 int num_sms) {
+  if constexpr (mid_bra_possible<LC, LD, R>())
+    if (mid_bra(blk.bra.la, blk.bra.lb, LD))
+      return launch_range_at<LC, LD, F0, F1, R, true>(blk, args, tab, stream, num_sms);
+  return launch_range_at<LC, LD, F0, F1, R, false>(blk, args, tab, stream, num_sms);
 }
 
 // The n blocks of a list (device memory; one bra (la, lb), Pmax the most primitive quartets
@@ -645,17 +788,10 @@ int launch_range(const QuartetBlock& blk, const JKArgs& args, const RysTablesVie
 template <int LC, int LD, int F0, int F1>
 int launch_range_list(int la, int lb, int64_t Pmax, const MultiEntry* list, int n, int64_t nwork, const JKArgs& args,
                       const RysTablesView& tab, cudaStream_t stream, int num_sms) {
-  BlockGeom g;
-  int threads;
-  size_t smem;
-  const int per_sm = block_geometry<LC, LD, F0, F1, double>(la, lb, Pmax, &g, &threads, &smem);
-  if (per_sm < 0) return per_sm;
-  const int64_t slots = (int64_t)num_sms * per_sm;
-  g.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, nwork / (slots * 8)));
-  const int64_t want = (nwork + g.chunk - 1) / g.chunk;
-  eri_block_kernel<LC, LD, F0, F1, double><<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(
-      QuartetBlock{}, args, tab, g, 1, 1, list, n, nwork);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  if constexpr (mid_bra_possible<LC, LD, double>())
+    if (mid_bra(la, lb, LD))
+      return launch_range_list_at<LC, LD, F0, F1, true>(la, lb, Pmax, list, n, nwork, args, tab, stream, num_sms);
+  return launch_range_list_at<LC, LD, F0, F1, false>(la, lb, Pmax, list, n, nwork, args, tab, stream, num_sms);
 }
 
 }  // namespace block_detail

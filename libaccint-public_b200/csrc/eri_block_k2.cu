@@ -5,9 +5,9 @@
 namespace lai {
 namespace block_detail {
 
-template int launch_range<2, 2, 2, 4, double>(const QuartetBlock&, const JKArgs&,
+template int launch_range<2, 2, 0, 4, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
-template int launch_range_list<2, 2, 2, 4>(int, int, int64_t, const MultiEntry*, int, int64_t,
+template int launch_range_list<2, 2, 0, 4>(int, int, int64_t, const MultiEntry*, int, int64_t,
                                           const JKArgs&, const RysTablesView&, cudaStream_t, int);
 template int launch_range<2, 2, 2, 4, float>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);

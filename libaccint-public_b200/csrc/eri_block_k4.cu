@@ -5,9 +5,9 @@
 namespace lai {
 namespace block_detail {
 
-template int launch_range<3, 3, 3, 6, double>(const QuartetBlock&, const JKArgs&,
+template int launch_range<3, 3, 0, 6, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
-template int launch_range_list<3, 3, 3, 6>(int, int, int64_t, const MultiEntry*, int, int64_t,
+template int launch_range_list<3, 3, 0, 6>(int, int, int64_t, const MultiEntry*, int, int64_t,
                                           const JKArgs&, const RysTablesView&, cudaStream_t, int);
 template int launch_range<3, 3, 3, 6, float>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);

@@ -5,9 +5,9 @@
 namespace lai {
 namespace block_detail {
 
-template int launch_range<4, 2, 4, 6, double>(const QuartetBlock&, const JKArgs&,
+template int launch_range<4, 2, 0, 6, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
-template int launch_range_list<4, 2, 4, 6>(int, int, int64_t, const MultiEntry*, int, int64_t,
+template int launch_range_list<4, 2, 0, 6>(int, int, int64_t, const MultiEntry*, int, int64_t,
                                           const JKArgs&, const RysTablesView&, cudaStream_t, int);
 
 }  // namespace block_detail

@@ -5,9 +5,9 @@
 namespace lai {
 namespace block_detail {
 
-template int launch_range<4, 3, 4, 5, double>(const QuartetBlock&, const JKArgs&,
+template int launch_range<4, 3, 0, 5, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);
-template int launch_range_list<4, 3, 4, 5>(int, int, int64_t, const MultiEntry*, int, int64_t,
+template int launch_range_list<4, 3, 0, 5>(int, int, int64_t, const MultiEntry*, int, int64_t,
                                           const JKArgs&, const RysTablesView&, cudaStream_t, int);
 template int launch_range<4, 3, 6, 7, double>(const QuartetBlock&, const JKArgs&,
                                              const RysTablesView&, cudaStream_t, int);

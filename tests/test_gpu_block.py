@@ -61,3 +61,23 @@ def test_block_kernel_equals_host_digestion(shells):
     # the sum (recurrences with both signs)
     assert np.max(np.abs(Jm - Jh)) < 1e-5 * np.max(np.abs(Jh))
     assert np.max(np.abs(Km - Kh)) < 1e-5 * np.max(np.abs(Kh))
+
+
+@pytest.mark.parametrize("ls", [(2,), (3,), (2, 3), (3, 4)])
+def test_transfer_on_both_sides_keeps_precision(ls):
+    """d, f and g shells on three centres: the transfer of (ff|ff) and its neighbours, done
+    once per quartet, must not lose what doing it per root keeps (the raw integrals' kernel)."""
+    rng = np.random.default_rng(3)
+    Z, xyz = lai.molecules.water_cluster_n(1, rng)
+    basis = lai.BasisSet([s for s in lai.BasisSet.from_atoms(Z, xyz, "cc-pvqz").shells if s.l in ls])
+    n = basis.nbf
+    C = rng.normal(size=(n, 5)) / np.sqrt(n)
+    D = C @ C.T
+    eng = lai.Engine(basis, threshold=0.0)
+    J, K, _ = eng.jk(D)
+    Jh, Kh = _host_jk(eng, n, D)
+    # both routes round some hundred terms per element to 1e-16, their errors independent:
+    # 2e-15 of the norm, 7e-15 in the d shells' K, small by cancellation in D.  Transferred
+    # about the first shell's centre on both sides, K' of (3,) is off by 4e-14
+    assert np.linalg.norm(J - Jh) < 5e-15 * np.linalg.norm(Jh)
+    assert np.linalg.norm(K - Kh) < 1e-14 * np.linalg.norm(Kh)
