@@ -6,10 +6,10 @@
 namespace lai {
 namespace grad_block {
 #define LAI_GRAD_KETS(K) \
-  K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 2, 4) K(3, 0, 3, 3) \
-  K(3, 1, 3, 4) K(3, 2, 3, 4) K(3, 2, 5, 5) K(3, 3, 3, 4) K(3, 3, 5, 5) K(3, 3, 6, 6) K(4, 0, 4, 4) \
-  K(4, 1, 4, 5) K(4, 2, 4, 5) K(4, 2, 6, 6) K(4, 3, 4, 5) K(4, 3, 6, 6) K(4, 3, 7, 7) K(4, 4, 4, 5) \
-  K(4, 4, 6, 6) K(4, 4, 7, 7) K(4, 4, 8, 8)
+  K(0, 0, 0, 0) K(1, 0, 1, 1) K(1, 1, 1, 2) K(2, 0, 2, 2) K(2, 1, 2, 3) K(2, 2, 0, 4) K(3, 0, 3, 3) \
+  K(3, 1, 3, 4) K(3, 2, 0, 4) K(3, 2, 5, 5) K(3, 3, 0, 4) K(3, 3, 5, 5) K(3, 3, 6, 6) K(4, 0, 4, 4) \
+  K(4, 1, 4, 5) K(4, 2, 0, 4) K(4, 2, 5, 5) K(4, 2, 6, 6) K(4, 3, 4, 5) K(4, 3, 6, 6) K(4, 3, 7, 7) \
+  K(4, 4, 4, 5) K(4, 4, 6, 6) K(4, 4, 7, 7) K(4, 4, 8, 8)
 #define K(c, d, f0, f1)                                                                                    \
   extern template int launch_grad_range<c, d, f0, f1>(const QuartetBlock&, const GradBlockArgs&,          \
                                                       const RysTablesView&, cudaStream_t, int);

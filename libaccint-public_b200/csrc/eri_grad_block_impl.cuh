@@ -19,6 +19,20 @@
 // quartet and root, and combining nine products per integral, this leaves about three times
 // the work of the J/K kernel.
 //
+// Where A (or C) lies far from the charge the terms of the transfer are large and cancel, and
+// with both sides transferred once per quartet the factors multiply (eri_block_impl.cuh).
+// So the bras that are there, (dd| against (dd| and larger kets (template parameter BM), and
+// the kets (dd|, (fd|, (ff| and (gd| are expanded about M, the centre P of the pair's first
+// primitive.  With u = x - M + (M-A),
+//   d/dA_x: 2 alpha ((e+1x 0|f0) + (M-A)_x (e0|f0)) contracted with W, less the contraction
+// of dW/d(M-A)_x with G; the same for C and D with their own exponents.  Error of the
+// gradient of H2O/cc-pVQZ's f shells alone, four geometries: 3e-14 to 1e-13 of its norm about
+// A and C, 1.4e-15 to 3.1e-15 about M (the kernel that transferred per primitive quartet:
+// 2.6e-15 to 6.7e-15); d shells 5e-15 to 1e-14, 9e-16 to 2.2e-15 (1.4e-15 to 5.8e-15).
+// (H2O)6/cc-pVDZ gradient 11.46 -> 11.45 ms.  The kets (gf| and (gg| stay about C: their
+// unrolled derivatives would be 25000 and 50000 products, and with the bra about M the error
+// with g shells is 1e-15 to 4.5e-15.
+//
 // A ket's f shells are split over launches (F0..F1) where W and G do not fit the
 // registers; every term is linear in W.
 #pragma once
@@ -30,7 +44,8 @@ namespace grad_block {
 
 using namespace block_detail;
 
-constexpr int kMaxThreadsGrad = kMaxThreads;
+template <int LC, int LD>
+__host__ __device__ constexpr bool grad_mid_ket() { return LD >= 2 && LC + LD <= 6; }
 
 struct GradBlockArgs {
   const double* D;
@@ -57,17 +72,28 @@ constexpr int transfer_terms(int l) {  // sum over the components of shell l of 
   return n;
 }
 
-template <int LC, int LD>
+// the same about M: sum over a and b of prod (a_x + b_x + 1)
+inline int mid_transfer_terms(int la, int lb) {
+  int n = 0;
+  for (int a = 0; a < ncart(la); ++a)
+    for (int b = 0; b < ncart(lb); ++b) {
+      const int ca = cart_comp(la, a), cb = cart_comp(lb, b);
+      n += (comp_x(ca) + comp_x(cb) + 1) * (comp_y(ca) + comp_y(cb) + 1) * (comp_z(ca) + comp_z(cb) + 1);
+    }
+  return n;
+}
+
+template <int LC, int LD, bool BM>
 __host__ GradBlockGeom make_grad_block_geom(int la, int lb, int threads, int batch) {
   constexpr int WS = odd_stride(LC + LD + 2), ND = ncart(LD), NC = ncart(LC);
   constexpr int NVP = odd_stride(chunk_components(LC, LD) * ND);
   GradBlockGeom g{};
   g.la = la; g.lb = lb;
   g.nroots = (la + lb + LC + LD + 1) / 2 + 1;
-  g.ne = ncart_range(la, la + lb);
+  g.ne = ncart_range(BM ? 0 : la, la + lb);
   g.na = ncart(la); g.nb = ncart(lb); g.nab = g.na * g.nb;
   g.nacc = g.nab + NC * ND + g.na * NC + g.na * ND + g.nb * NC + g.nb * ND;
-  g.nentry = g.na * transfer_terms(lb);
+  g.nentry = BM ? mid_transfer_terms(la, lb) : g.na * transfer_terms(lb);
   g.batch = batch;
   g.ts = (la + lb + 2) * WS;
   int o = 0;
@@ -75,8 +101,9 @@ __host__ GradBlockGeom make_grad_block_geom(int la, int lb, int threads, int bat
   g.o_tab = take(batch * g.nroots * 3 * g.ts);
   g.o_v = take(g.nab * NVP);
   g.o_d = take(g.nacc);
-  g.o_cob = take(4 * g.nb * kMaxTerms);  // coefficients, then their derivatives by AB_x
-  g.o_cod = take(4 * ND * kMaxTerms);
+  // coefficients, then their derivatives by AB_x (BM: by M-A in the same direction)
+  g.o_cob = take(BM ? 6 * (la + 1) * (lb + 1) * (la + lb + 1) : 4 * g.nb * kMaxTerms);
+  g.o_cod = take(grad_mid_ket<LC, LD>() ? 3 * (LC + 1) * (LD + 1) * (LC + LD + 1) : 4 * ND * kMaxTerms);
   g.o_nab = take(g.nab);
   g.o_ncd = take(NC * ND);
   g.o_exp = take(3 * batch);             // alpha, gamma, delta of every batched primitive quartet
@@ -87,9 +114,10 @@ __host__ GradBlockGeom make_grad_block_geom(int la, int lb, int threads, int bat
   return g;
 }
 
-template <int LC, int LD, int F0, int F1>
-__global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBlock blk, GradBlockArgs ga,
-                                                                     RysTablesView tab, GradBlockGeom g) {
+template <int LC, int LD, int F0, int F1, bool BM>
+__global__ void __launch_bounds__((BM ? kMaxThreadsMid : kMaxThreads))
+    grad_block_kernel(QuartetBlock blk, GradBlockArgs ga, RysTablesView tab, GradBlockGeom g) {
+  constexpr bool KM = grad_mid_ket<LC, LD>();
   constexpr int LCD = LC + LD, WS = odd_stride(LCD + 2);
   constexpr int NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
   constexpr int CB = chunk_components(LC, LD), NV = CB * ND, NVP = odd_stride(NV);
@@ -112,7 +140,8 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
   double* const Ncd = smem_g + g.o_ncd;
   double* const Ex = smem_g + g.o_exp;
   int64_t* const list = reinterpret_cast<int64_t*>(smem_g + g.o_int);
-  int* const entry = reinterpret_cast<int*>(list + nt);  // by row e: ab | (b kMaxTerms + term) << 16
+  // by row e: ab | (b kMaxTerms + term) << 16, or (BM) ab | (a_x, b_x) << 8 | (a_y, b_y) << 13 | (a_z, b_z) << 18
+  int* const entry = reinterpret_cast<int*>(list + nt);
   int* const first = entry + g.nentry;                   // [NE + 1] first entry of each row
   int* const fill = first + NE + 1;
   int* const bc = fill + NE + 1;
@@ -132,6 +161,15 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
     const int ca = cart_comp(la, a), cb = cart_comp(lb, b);
     const int bx = comp_x(cb), by = comp_y(cb), bz = comp_z(cb);
     int t = 0;
+    if constexpr (BM) {
+      const int ax = comp_x(ca), ay = comp_y(ca), az = comp_z(ca);
+      const int pairs = (ax * (lb + 1) + bx) | ((ay * (lb + 1) + by) << 5) | ((az * (lb + 1) + bz) << 10);
+      for (int kx = 0; kx <= ax + bx; ++kx)
+        for (int ky = 0; ky <= ay + by; ++ky)
+          for (int kz = 0; kz <= az + bz; ++kz)
+            f(0, ncart_before(0, kx + ky + kz) + cart_index(kx, ky, kz), 0, pairs);
+      return;
+    }
     for (int kx = 0; kx <= bx; ++kx)
       for (int ky = 0; ky <= by; ++ky)
         for (int kz = 0; kz <= bz; ++kz, ++t)
@@ -142,7 +180,7 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
   for (int i = tid; i < NAB; i += nt) {
     each_term(i, [&](int t, int e, int c, int pw) {
       atomicAdd(first + e + 1, 1);
-      if (i < NB) {
+      if (!BM && i < NB) {
         bc[i * kMaxTerms + t] = c;
         bp[i * kMaxTerms + t] = pw;
       }
@@ -151,7 +189,7 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
   }
   for (int i = tid; i < NCD; i += nt) {
     Ncd[i] = norm_factor(LC, i / ND) * norm_factor(LD, i % ND);
-    if (i < ND) {
+    if (!KM && i < ND) {
       const int cd = cart_comp(LD, i);
       const int dx = comp_x(cd), dy = comp_y(cd), dz = comp_z(cd);
       int t = 0;
@@ -180,13 +218,13 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
     for (int e = 0; e < NE; ++e) first[e + 1] += first[e];
   __syncthreads();
   for (int i = tid; i < NAB; i += nt)
-    each_term(i, [&](int t, int e, int, int) {
-      entry[first[e] + atomicAdd(fill + e, 1)] = i | (((i % NB) * kMaxTerms + t) << 16);
+    each_term(i, [&](int t, int e, int, int pw) {
+      entry[first[e] + atomicAdd(fill + e, 1)] = BM ? i | (pw << 8) : i | (((i % NB) * kMaxTerms + t) << 16);
     });
   // this thread's rows of the tables, and its component
   int ox = 0, oy = g.ts, oz = 2 * g.ts, ex = 0, ey = 0, ez = 0;
   if (tid < NE) {
-    int l = la, r = tid;
+    int l = BM ? 0 : la, r = tid;
     while (r >= ncart(l)) r -= ncart(l++);
     const int ce = cart_comp(l, r);
     ex = comp_x(ce); ey = comp_y(ce); ez = comp_z(ce);
@@ -219,6 +257,8 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
       const int fc = __ldg(blk.ket.func_a + q), fd = __ldg(blk.ket.func_b + q);
       const double sym = quartet_weight(blk, p, q);
       const double CD[3] = {__ldg(blk.ket.AB + q), __ldg(blk.ket.AB + nket + q), __ldg(blk.ket.AB + 2 * nket + q)};
+      const double* __restrict__ pbra = blk.bra.primb + (size_t)p * Kab * kBraRec;
+      const double* __restrict__ pket = blk.ket.primb + (size_t)q * Kcd * kBraRec;
       {  // density blocks; transfer coefficients C(b,k) AB^(b-k) and their derivatives
         const double* __restrict__ D = ga.D;
         auto func = [&](int sh) { return sh == 0 ? fa : sh == 1 ? fb : sh == 2 ? fc : fd; };
@@ -227,7 +267,27 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
           copy_async8(Dab + i, D + (size_t)(func(k & 3) + ((k >> 4) & 255)) * n + func((k >> 2) & 3) + (k >> 12));
         }
         const double AB[3] = {__ldg(blk.bra.AB + p), __ldg(blk.bra.AB + nbra + p), __ldg(blk.bra.AB + 2 * nbra + p)};
-        for (int i = tid; i < sB + sD; i += nt) {
+        if constexpr (BM) {
+          const int per = (la + 1) * (lb + 1), S = la + lb + 1;
+          for (int i = tid; i < 3 * per; i += nt) {
+            const int x = i / per, ij = i - x * per, ia = ij / (lb + 1), jb = ij - ia * (lb + 1);
+            const double ma = __ldg(pbra + BR_PAX + x), mb = ma + (x == 0 ? AB[0] : x == 1 ? AB[1] : AB[2]);
+            mid_coefs<kMaxLab + 1>(ma, mb, ia, jb, CoB + i * S);
+            double* d = CoB + (3 * per + i) * S;  // ia times the coefficients of one power less
+            if (ia) mid_coefs<kMaxLab + 1>(ma, mb, ia - 1, jb, d);
+            for (int k = 0; k < ia + jb; ++k) d[k] = ia ? ia * d[k] : 0.0;
+            d[ia + jb] = 0.0;
+          }
+        }
+        if constexpr (KM) {
+          constexpr int per = (LC + 1) * (LD + 1), S = LCD + 1;
+          for (int i = nt - 1 - tid; i < 3 * per; i += nt) {
+            const int x = i / per, ij = i - x * per, ic = ij / (LD + 1);
+            const double mc = __ldg(pket + BR_PAX + x), md = mc + (x == 0 ? CD[0] : x == 1 ? CD[1] : CD[2]);
+            mid_coefs<S>(mc, md, ic, ij - ic * (LD + 1), CoD + i * S);
+          }
+        }
+        for (int i = tid + (BM ? sB : 0); i < (KM ? sB : sB + sD); i += nt) {
           const bool bra = i < sB;
           const int j = bra ? i : i - sB;
           const int k = bra ? bp[j] : dp[j], m[3] = {k & 15, (k >> 4) & 15, k >> 8};
@@ -268,14 +328,22 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
         }
       };
       // row e of the bra-transposed chunk: out[cd] = sum over the row's terms of
-      // co[term] Gamma[ab][cd]
-      auto gather_row = [&](const double* co, double (&out)[NVP]) {
+      // coefficient * Gamma[ab][cd]; dir = 0, 1, 2: the coefficients' derivative by AB_x
+      // (BM: by (M-A)_x), 3: the coefficients
+      auto gather_row = [&](int dir, double (&out)[NVP]) {
+        const int S = la + lb + 1, per = (la + 1) * (lb + 1) * S;
+        const double* cx = CoB + (dir == 0 ? 3 * per : 0) + ex;
+        const double* cy = CoB + (dir == 1 ? 4 * per : per) + ey;
+        const double* cz = CoB + (dir == 2 ? 5 * per : 2 * per) + ez;
+        const double* co = CoB + (dir == 3 ? 0 : (dir + 1) * sB);
 #pragma unroll
         for (int j = 0; j < NV; ++j) out[j] = 0.0;
         for (int k = e_first; k < e_last; ++k) {
           const int en = entry[k];
-          const double c = co[en >> 16];
-          const double* v = Vs + (en & 0xffff) * NVP;
+          double c;
+          if constexpr (BM) c = cx[((en >> 8) & 31) * S] * cy[((en >> 13) & 31) * S] * cz[((en >> 18) & 31) * S];
+          else c = co[en >> 16];
+          const double* v = Vs + (en & (BM ? 0xff : 0xffff)) * NVP;
 #pragma unroll
           for (int j = 0; j < (NV + 1) / 2; ++j) {
             const double2 x = *reinterpret_cast<const double2*>(v + 2 * j);
@@ -283,6 +351,11 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
             if (2 * j + 1 < NV) out[2 * j + 1] += c * x.y;
           }
         }
+      };
+
+      // coefficients of (x-M + M-C)^i (x-M + M-D)^j in one direction (KM)
+      auto ket_co = [&](int x, int i, int j) {
+        return CoD + ((x * (LC + 1) + i) * (LD + 1) + j) * (LCD + 1);
       };
 
       // ---- W[e][f] ----
@@ -294,13 +367,31 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
         __syncthreads();
         if (tid < NE) {
           double row[NVP];
-          gather_row(CoB, row);
+          gather_row(3, row);
           bfor<0, NC / CB>([&](auto CH) {
             constexpr int c0_ = decltype(CH)::value * CB;
             if (c0 == c0_) {
               bfor<0, NV>([&](auto II) {
                 constexpr int i = decltype(II)::value;
                 constexpr int cc = cart_comp(LC, c0_ + i / ND), d = i % ND, cd = cart_comp(LD, d);
+                if constexpr (KM) {
+                  bfor<0, comp_x(cc) + comp_x(cd) + 1>([&](auto KX) {
+                    bfor<0, comp_y(cc) + comp_y(cd) + 1>([&](auto KY) {
+                      constexpr int kx = decltype(KX)::value, ky = decltype(KY)::value;
+                      constexpr int z0 = F0 - kx - ky > 0 ? F0 - kx - ky : 0;
+                      constexpr int mz = comp_z(cc) + comp_z(cd), z1 = mz < F1 - kx - ky ? mz : F1 - kx - ky;
+                      if constexpr (z0 <= z1) {
+                        const double w = row[i] * (ket_co(0, comp_x(cc), comp_x(cd))[kx] *
+                                                   ket_co(1, comp_y(cc), comp_y(cd))[ky]);
+                        bfor<z0, z1 + 1>([&](auto KZ) {
+                          constexpr int kz = decltype(KZ)::value;
+                          Wt[ncart_before(F0, kx + ky + kz) + cart_index(kx, ky, kz)] +=
+                              w * ket_co(2, comp_z(cc), comp_z(cd))[kz];
+                        });
+                      }
+                    });
+                  });
+                } else
                 bfor<0, comp_x(cd) + 1>([&](auto KX) {
                   bfor<0, comp_y(cd) + 1>([&](auto KY) {
                     bfor<0, comp_z(cd) + 1>([&](auto KZ) {
@@ -324,8 +415,6 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
 
       // ---- primitive quartets ----
       double gA[3] = {0.0, 0.0, 0.0}, gC[3] = {0.0, 0.0, 0.0}, gD[3] = {0.0, 0.0, 0.0};
-      const double* __restrict__ pbra = blk.bra.primb + (size_t)p * Kab * kBraRec;
-      const double* __restrict__ pket = blk.ket.primb + (size_t)q * Kcd * kBraRec;
       for (int64_t c0 = split; c0 < P; c0 += (int64_t)nt * g.nsplit) {
         int cnt;
         if (P == 1) {
@@ -372,7 +461,10 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
             double u, w;
             rys_root_one<double>(NR, r, T, tab, u, w);
             const double pqx = x == 0 ? PQx : x == 1 ? PQy : PQz;
-            const double pa = __ldg(pb + BR_PAX + x) - rz * u * pqx, qc = __ldg(pk + BR_PAX + x) + re * u * pqx;
+            // P - A and Q - C, or P - M and Q - M (0 in the first primitive)
+            const double pc = BM ? __ldg(pb + BR_PX + x) - __ldg(pbra + BR_PX + x) : __ldg(pb + BR_PAX + x);
+            const double qd = KM ? __ldg(pk + BR_PX + x) - __ldg(pket + BR_PX + x) : __ldg(pk + BR_PAX + x);
+            const double pa = pc - rz * u * pqx, qc = qd + re * u * pqx;
             const double b00 = 0.5 * inv * u, b10 = hz - hz * rz * u, b01 = he - he * re * u;
             double* dst = Tb + (size_t)(s * NR * 3 + rx) * g.ts;
             constexpr int E = kMaxLab + 1;
@@ -452,12 +544,12 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
 #pragma unroll
                   for (int j = 0; j <= F1; ++j) {
                     a += Pf[j] * hi[j];
-                    b += Pf[j] * lw[j];
+                    if (!BM) b += Pf[j] * lw[j];
                     uc_ += Pf[j] * I[j + 1];
-                    if (j) lc_ += Pf[j] * (j * I[j > 0 ? j - 1 : 0]);
+                    if (!KM && j) lc_ += Pf[j] * (j * I[j > 0 ? j - 1 : 0]);
                   }
                   u_ += a;
-                  l_ += e * b;
+                  if (!BM) l_ += e * b;
                 };
                 dir(Px, X, ox, ex, up[0], lo[0], uc[0], lc[0]);
                 dir(Py, Y, oy, ey, up[1], lo[1], uc[1], lc[1]);
@@ -468,9 +560,16 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
               const double al2 = 2.0 * Ex[3 * s], ga2 = 2.0 * Ex[3 * s + 1], de2 = 2.0 * Ex[3 * s + 2];
 #pragma unroll
               for (int x = 0; x < 3; ++x) {
-                gA[x] += al2 * up[x] - lo[x];
-                gC[x] += ga2 * uc[x] - lc[x];
-                gD[x] += de2 * (uc[x] + CD[x] * S);
+                if constexpr (BM) gA[x] += al2 * (up[x] + __ldg(pbra + BR_PAX + x) * S);
+                else gA[x] += al2 * up[x] - lo[x];
+                if constexpr (KM) {
+                  const double mc = __ldg(pket + BR_PAX + x);
+                  gC[x] += ga2 * (uc[x] + mc * S);
+                  gD[x] += de2 * (uc[x] + (mc + CD[x]) * S);
+                } else {
+                  gC[x] += ga2 * uc[x] - lc[x];
+                  gD[x] += de2 * (uc[x] + CD[x] * S);
+                }
               }
             }
           }
@@ -478,15 +577,16 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
         }
       }
 
-      // ---- the dependence of W on AB and CD, from the contracted G ----
-      double tAB[3] = {0.0, 0.0, 0.0}, tCD[3] = {0.0, 0.0, 0.0};
+      // ---- the dependence of W on AB and CD (about M: on M-A, M-C and M-D), from the
+      // contracted G ----
+      double tAB[3] = {0.0, 0.0, 0.0}, tCD[3] = {0.0, 0.0, 0.0}, tD[3] = {0.0, 0.0, 0.0};
       if (LD > 0 || lb > 0)
         for (int c0 = 0; c0 < NC; c0 += CB) {
           gamma_chunk(c0);
           __syncthreads();
           if (tid < NE) {
             double H[NV], row[NVP];
-            gather_row(CoB, row);
+            gather_row(3, row);
             bfor<0, NC / CB>([&](auto CH) {
               constexpr int c0_ = decltype(CH)::value * CB;
               if (c0 == c0_) {
@@ -494,6 +594,42 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
                   constexpr int i = decltype(II)::value;
                   constexpr int cc = cart_comp(LC, c0_ + i / ND), d = i % ND, cd = cart_comp(LD, d);
                   double h = 0.0;
+                  if constexpr (KM) {
+                    constexpr int c_x = comp_x(cc), c_y = comp_y(cc), c_z = comp_z(cc);
+                    constexpr int d_x = comp_x(cd), d_y = comp_y(cd), d_z = comp_z(cd);
+                    double hc[3] = {0.0, 0.0, 0.0}, hd[3] = {0.0, 0.0, 0.0};
+                    bfor<0, c_x + d_x + 1>([&](auto KX) {
+                      bfor<0, c_y + d_y + 1>([&](auto KY) {
+                        constexpr int kx = decltype(KX)::value, ky = decltype(KY)::value;
+                        constexpr int z0 = F0 - kx - ky > 0 ? F0 - kx - ky : 0;
+                        constexpr int mz = c_z + d_z, z1 = mz < F1 - kx - ky ? mz : F1 - kx - ky;
+                        if constexpr (z0 <= z1) {
+                          double sz = 0.0, sc = 0.0, sd = 0.0;  // over z: coefficients, derivatives by M-C and M-D
+                          bfor<z0, z1 + 1>([&](auto KZ) {
+                            constexpr int kz = decltype(KZ)::value;
+                            const double gf = G[ncart_before(F0, kx + ky + kz) + cart_index(kx, ky, kz)];
+                            sz += ket_co(2, c_z, d_z)[kz] * gf;
+                            if constexpr (c_z > 0 && kz < mz) sc += ket_co(2, c_z - 1, d_z)[kz] * gf;
+                            if constexpr (d_z > 0 && kz < mz) sd += ket_co(2, c_z, d_z - 1)[kz] * gf;
+                          });
+                          const double cx = ket_co(0, c_x, d_x)[kx], cy = ket_co(1, c_y, d_y)[ky];
+                          h += cx * cy * sz;
+                          hc[2] += cx * cy * sc;
+                          hd[2] += cx * cy * sd;
+                          if constexpr (c_x > 0 && kx < c_x + d_x) hc[0] += ket_co(0, c_x - 1, d_x)[kx] * (cy * sz);
+                          if constexpr (d_x > 0 && kx < c_x + d_x) hd[0] += ket_co(0, c_x, d_x - 1)[kx] * (cy * sz);
+                          if constexpr (c_y > 0 && ky < c_y + d_y) hc[1] += ket_co(1, c_y - 1, d_y)[ky] * (cx * sz);
+                          if constexpr (d_y > 0 && ky < c_y + d_y) hd[1] += ket_co(1, c_y, d_y - 1)[ky] * (cx * sz);
+                        }
+                      });
+                    });
+                    if constexpr (c_x > 0) tCD[0] += row[i] * (c_x * hc[0]);
+                    if constexpr (c_y > 0) tCD[1] += row[i] * (c_y * hc[1]);
+                    if constexpr (c_z > 0) tCD[2] += row[i] * (c_z * hc[2]);
+                    if constexpr (d_x > 0) tD[0] += row[i] * (d_x * hd[0]);
+                    if constexpr (d_y > 0) tD[1] += row[i] * (d_y * hd[1]);
+                    if constexpr (d_z > 0) tD[2] += row[i] * (d_z * hd[2]);
+                  } else
                   bfor<0, comp_x(cd) + 1>([&](auto KX) {
                     bfor<0, comp_y(cd) + 1>([&](auto KY) {
                       bfor<0, comp_z(cd) + 1>([&](auto KZ) {
@@ -520,7 +656,7 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
             if (lb > 0) {
 #pragma unroll
               for (int x = 0; x < 3; ++x) {
-                gather_row(CoB + (x + 1) * sB, row);
+                gather_row(x, row);
 #pragma unroll
                 for (int j = 0; j < NV; ++j) tAB[x] += row[j] * H[j];
               }
@@ -533,9 +669,9 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
       double v[9];
 #pragma unroll
       for (int x = 0; x < 3; ++x) {
-        v[x] = gA[x] + tAB[x];
-        v[3 + x] = gC[x] + tCD[x];
-        v[6 + x] = gD[x] - tCD[x];
+        v[x] = BM ? gA[x] - tAB[x] : gA[x] + tAB[x];
+        v[3 + x] = KM ? gC[x] - tCD[x] : gC[x] + tCD[x];
+        v[6 + x] = KM ? gD[x] - tD[x] : gD[x] - tCD[x];
       }
 #pragma unroll
       for (int i = 0; i < 9; ++i)
@@ -559,19 +695,18 @@ __global__ void __launch_bounds__(kMaxThreadsGrad) grad_block_kernel(QuartetBloc
   }
 }
 
-// 0 when launched, -3 on a CUDA error.
-template <int LC, int LD, int F0, int F1>
-int launch_grad_range(const QuartetBlock& blk, const GradBlockArgs& ga, const RysTablesView& tab, cudaStream_t stream,
+template <int LC, int LD, int F0, int F1, bool BM>
+int launch_grad_range_at(const QuartetBlock& blk, const GradBlockArgs& ga, const RysTablesView& tab, cudaStream_t stream,
                       int num_sms) {
   const int la = blk.bra.la, lb = blk.bra.lb;
-  const int threads = (ncart_range(la, la + lb) + 31) / 32 * 32;
+  const int threads = (ncart_range(BM ? 0 : la, la + lb) + 31) / 32 * 32;
   const int nroots = (la + lb + LC + LD + 1) / 2 + 1;
   const int64_t P = (int64_t)blk.bra.Ka * blk.bra.Kb * blk.ket.Ka * blk.ket.Kb;
   int batch = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(P, 8), threads / (3 * nroots)));
-  GradBlockGeom g = make_grad_block_geom<LC, LD>(la, lb, threads, batch);
-  while (g.doubles * 8 > kMaxSmem && batch > 1) g = make_grad_block_geom<LC, LD>(la, lb, threads, --batch);
+  GradBlockGeom g = make_grad_block_geom<LC, LD, BM>(la, lb, threads, batch);
+  while (g.doubles * 8 > kMaxSmem && batch > 1) g = make_grad_block_geom<LC, LD, BM>(la, lb, threads, --batch);
   const size_t smem = sizeof(double) * (size_t)g.doubles;
-  auto kern = grad_block_kernel<LC, LD, F0, F1>;
+  auto kern = grad_block_kernel<LC, LD, F0, F1, BM>;
   static std::atomic<int> occ[kMaxL + 1][kMaxL + 1][9];
   int per_sm = occ[la][lb][batch].load(std::memory_order_relaxed);
   if (per_sm == 0) {
@@ -588,6 +723,16 @@ int launch_grad_range(const QuartetBlock& blk, const GradBlockArgs& ga, const Ry
   const int64_t want = (nwork + g.chunk - 1) / g.chunk;
   kern<<<(unsigned)std::min<int64_t>(want, slots), threads, smem, stream>>>(blk, ga, tab, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// 0 when launched, -3 on a CUDA error.
+template <int LC, int LD, int F0, int F1>
+int launch_grad_range(const QuartetBlock& blk, const GradBlockArgs& ga, const RysTablesView& tab, cudaStream_t stream,
+                      int num_sms) {
+  if constexpr (mid_bra_possible<LC, LD, double>())
+    if (mid_bra(blk.bra.la, blk.bra.lb, LD) || (LD == 2 && blk.bra.lb == 2))
+      return launch_grad_range_at<LC, LD, F0, F1, true>(blk, ga, tab, stream, num_sms);
+  return launch_grad_range_at<LC, LD, F0, F1, false>(blk, ga, tab, stream, num_sms);
 }
 
 }  // namespace grad_block

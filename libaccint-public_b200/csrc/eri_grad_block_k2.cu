@@ -5,7 +5,7 @@
 namespace lai {
 namespace grad_block {
 
-template int launch_grad_range<2, 2, 2, 4>(const QuartetBlock&, const GradBlockArgs&,
+template int launch_grad_range<2, 2, 0, 4>(const QuartetBlock&, const GradBlockArgs&,
                                            const RysTablesView&, cudaStream_t, int);
 
 }  // namespace grad_block

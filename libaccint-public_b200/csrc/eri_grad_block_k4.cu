@@ -5,7 +5,7 @@
 namespace lai {
 namespace grad_block {
 
-template int launch_grad_range<3, 2, 3, 4>(const QuartetBlock&, const GradBlockArgs&,
+template int launch_grad_range<3, 2, 0, 4>(const QuartetBlock&, const GradBlockArgs&,
                                            const RysTablesView&, cudaStream_t, int);
 template int launch_grad_range<3, 2, 5, 5>(const QuartetBlock&, const GradBlockArgs&,
                                            const RysTablesView&, cudaStream_t, int);

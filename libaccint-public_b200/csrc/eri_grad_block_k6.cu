@@ -5,7 +5,9 @@
 namespace lai {
 namespace grad_block {
 
-template int launch_grad_range<4, 2, 4, 5>(const QuartetBlock&, const GradBlockArgs&,
+template int launch_grad_range<4, 2, 0, 4>(const QuartetBlock&, const GradBlockArgs&,
+                                           const RysTablesView&, cudaStream_t, int);
+template int launch_grad_range<4, 2, 5, 5>(const QuartetBlock&, const GradBlockArgs&,
                                            const RysTablesView&, cudaStream_t, int);
 template int launch_grad_range<4, 2, 6, 6>(const QuartetBlock&, const GradBlockArgs&,
                                            const RysTablesView&, cudaStream_t, int);
