@@ -320,7 +320,9 @@ LAI_API int lai_sph_to_cart_density_device(lai_engine* engine, const double* d_D
  *              src/host/kernels/three_center_eri_kernel.cpp:273-362);
  *   lai_eri2c: V[P*naux + Q] = (P|Q) (compute_two_center_metric,
  *              src/host/kernels/two_center_coulomb_kernel.cpp:212-251).
- * Orbital shells up to f (g only paired with s), auxiliary shells up to g.  The
+ * Orbital shells up to f (g only paired with s), auxiliary shells up to g.  In T,
+ * primitive pairs whose product has a prefactor below exp(-80) (2e-35) are left out: an
+ * element made of such pairs alone is exactly 0.  The
  * _device variants write device buffers asynchronously on stream.
  * ------------------------------------------------------------------------- */
 LAI_API int lai_eri3c(lai_engine* engine, const lai_basis* aux, double* T);

@@ -661,7 +661,9 @@ __global__ void symmetrize_batched_kernel(const double* __restrict__ Jp, const d
 // H2O/cc-pVQZ 666 of them for 120 angular classes; a launch each leaves the device to
 // their set-up (lookup tables, class tables, 15 - 25 us of latency whatever the work).
 // The blocks of one angular class that do not fill the device alone go out as one launch,
-// each with its own split of a quartet, the heaviest items first.
+// each with its own split of a quartet, the heaviest items first.  Larger ones keep a launch
+// of their own: a list has one geometry for all its entries, the table batch of the longest
+// contraction, and holds its items together in time.
 int build_launches(lai_engine* E) {
   const int nb = (int)E->blocks.size();
   std::map<std::array<int, 5>, std::vector<int>> groups;  // kernel and class -> blocks
@@ -672,7 +674,8 @@ int build_launches(lai_engine* E) {
     int kind = 0;  // 1: thread-per-quartet, split; 2: block-per-quartet
     if (lai::small_class_supported(la, lb, lc, ld))
       kind = lai::block_for_few(q, E->num_sms) ? 2 : q.total < (int64_t)E->num_sms * lai::kSplitQuartetsPerSm ? 1 : 0;
-    else if (lai::default_kernel(la, lb, lc, ld, q.total, E->num_sms) == lai::KERNEL_BLOCK)
+    else if (lai::default_kernel(la, lb, lc, ld, q.total, E->num_sms) == lai::KERNEL_BLOCK &&
+             q.total < (int64_t)E->num_sms * lai::kListBlocksPerSm)
       kind = 2;
     if (kind) groups[{kind, la, lb, lc, ld}].push_back(b);
     else single.push_back(b);

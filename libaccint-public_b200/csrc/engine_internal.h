@@ -251,12 +251,14 @@ int ensure_accumulators(lai_engine* E, size_t elems);
 // the lane with the least estimated work so far; join() makes the caller's stream wait
 // for all of them.  The class-pair launches of one build only add to J'/K' (or the
 // gradient) with atomics, so their order does not matter, and most of them do not fill
-// the device alone: H2O / cc-pVQZ takes 666 launches, most with a few warps.  The blocks
+// the device alone: H2O / cc-pVQZ has 666 class pairs, most with work for a few warps.  The blocks
 // go out by descending estimated work, so that the small launches fill the large ones'
 // last waves.  kLanes is the number of hardware queues a process gets by default; more
-// streams would share them.  One stream -> eight (device time of a build): H2O/STO-3G
-// 106 -> 49 us, H2O/cc-pVQZ 320 -> 120 ms, (H2O)16/cc-pVDZ 53.2 -> 39.3 ms,
-// (H2O)64/cc-pVDZ 1505 -> 1390 ms; (H2O)6/cc-pVDZ gradient 82.5 -> 30.5 ms.
+// streams would share them.  One stream -> eight, with the kernels of the time (device time
+// of a build): H2O/STO-3G 106 -> 49 us, (H2O)16/cc-pVDZ 53.2 -> 39.3 ms, (H2O)64/cc-pVDZ
+// 1505 -> 1390 ms; (H2O)6/cc-pVDZ gradient 82.5 -> 30.5 ms.  Now, every launch by itself on
+// one stream against a build: H2O/cc-pVQZ 19.6 -> 3.3 ms (small launches shared as well),
+// C6H14/cc-pVTZ 90.6 -> 86.1 ms.
 class LaunchLanes {
  public:
   LaunchLanes(lai_engine* E, cudaStream_t stream, size_t lanes);

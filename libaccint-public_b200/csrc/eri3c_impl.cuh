@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(128) eri3c_kernel(Eri3cArgs g) {
     for (int ib = 0; ib < B.np; ++ib) {
       const double be = __ldg(g.exps + B.poff + ib), cb = __ldg(g.coefs + B.poff + ib);
       const double p = al + be, ip = 1.0 / p, arg = al * be * ip * r2;
-      // exp(-80) = 2e-35: no element can show it (tight functions of two atoms, half of the
+      // exp(-80) = 2e-35, far below the rounding of any element that other pairs reach; an
+      // element with no other pair is exactly 0 (tight functions of two atoms, half of the
       // primitive pairs of a cluster; the pair is the same for nearly all of a warp)
       if (arg > 80.0) continue;
       const double cab = ca * cb * exp(-arg);

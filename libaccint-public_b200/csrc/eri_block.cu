@@ -91,8 +91,9 @@ bool block_for_few(const QuartetBlock& blk, int num_sms) {
 // What the block kernel replaced in the other classes was the tiled kernel (one warp per
 // quartet, its table and digestion sweeps repeated for every 512 integrals) and a
 // warp-per-quartet kernel with scattered (e0|f0) ownership.  Device time per class,
-// C6H14/cc-pVTZ, before -> now: (fd|dp) 21.6 -> 1.9 ms, (fp|dp) 23.1 -> 2.6, (fd|dd) 10.3
-// -> 0.8, (ff|fd) 8.1 -> 0.3, (dd|dp) 6.2 -> 3.1; one (gg|gg) quartet 74 ms -> 0.1 ms.  Whole builds: C6H14/cc-pVTZ 199 -> 90 ms, H2O/cc-pVQZ 120 -> 5.1 ms.
+// C6H14/cc-pVTZ, before -> now: (fd|dp) 21.6 -> 2.7 ms, (fp|dp) 23.1 -> 3.2, (fd|dd) 10.3
+// -> 1.4, (ff|fd) 8.1 -> 0.4, (dd|dp) 6.2 -> 3.8; one (gg|gg) quartet 74 ms -> 0.07 ms.
+// Whole builds when it came: C6H14/cc-pVTZ 199 -> 90 ms, H2O/cc-pVQZ 120 -> 5.1 ms.
 int default_kernel(int la, int lb, int lc, int ld, int64_t nq, int num_sms) {
   if (nq >= (int64_t)32 * num_sms && sliced_class_supported(la, lb, lc, ld)) return KERNEL_SLICED;
   return KERNEL_BLOCK;

@@ -2,7 +2,7 @@
 // thread: compile-time specialised on the ket (lc, ld), any bra (la, lb).  J/K digestion
 // only (the raw-integral and Schwarz modes stay on the tiled kernel).
 //
-// One block of 32-160 threads per quartet; thread e owns row e of the contracted
+// One block of 32-192 threads per quartet; thread e owns row e of the contracted
 // (e0|f0) block, e over the Cartesian components of shells la..la+lb, and holds
 // G[f] for every component f of the ket shells F0..F1 in registers:
 //   1. table phase: for up to `batch` primitive quartets at once, one thread per
@@ -84,8 +84,8 @@ constexpr int kMaxSmem = 226 * 1024;  // of 227 KB, less the static part
 // 8 warps per SM, each waiting on its own arithmetic and shared-memory latency (ncu, (dd|dp):
 // issue active 30 %, stalls `wait` and `short_scoreboard`).  Caps of 96 and 128 registers
 // (65536 / (160 * blocks)) pay for the kets of few components, C6H14/cc-pVTZ without and
-// with them: (fd|ps) 4.9 -> 3.5 ms, (ff|ps) 1.6 -> 0.9, (fs|dp) 4.8 -> 4.0, (fd|pp) 1.75 ->
-// 1.67, but (dd|pp) 2.5 -> 2.8; from 25 components on the spills cost more ((dd|fp) 1.2 ->
+// with them: (fd|ps) 4.9 -> 3.5 ms, (ff|ps) 1.6 -> 0.9, (fs|dp) 4.8 -> 4.0, but (dd|pp) 2.5
+// -> 2.8; with the bra about M (fd|pp) 3.07 -> 2.79, (ff|pp) 1.26 -> 0.73; from 25 components on the spills cost more ((dd|fp) 1.2 ->
 // 1.6 with 128).
 template <int F0, int F1, bool BM>
 __host__ __device__ constexpr int min_blocks() {  // (BM: blocks of 192 threads, nearly the same caps)

@@ -33,6 +33,12 @@ struct MultiEntry {
 };
 // A launch with fewer quartets per SM than this splits them over lanes.
 constexpr int kSplitQuartetsPerSm = 1024;
+// A block-kernel launch with fewer quartets per SM than this shares a launch.  Without a
+// limit -> 1024 -> 256 -> 64 -> 16: C6H14/cc-pVTZ 84.4, 83.3, 81.7, 79.7, 79.5 ms, (H2O)2/cc-pVQZ
+// 27.3, 27.4, 27.4, 27.1, 26.5, (H2O)23/cc-pVDZ 91.5, 91.5, 89.8, 89.8, 89.8, (H2O)64/cc-pVDZ
+// 1318, 1306, 1307, 1307, 1308; below 16 the small ones wait for launches again
+// ((H2O)4/cc-pVTZ 13.6, 13.5, 13.6, 13.5, 13.7, (H2O)8/cc-pVDZ 5.13, 5.14, 5.14, 5.14, 5.17).
+constexpr int kListBlocksPerSm = 64;
 int launch_small_list(int la, int lb, int lc, int ld, const MultiEntry* list, int n, int64_t nwork,
                       const JKArgs& args, const RysTablesView& tab, cudaStream_t stream, int num_sms);
 int launch_small(const QuartetBlock& blk, const JKArgs& args, const RysTablesView& tab,

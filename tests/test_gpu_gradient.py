@@ -188,7 +188,7 @@ def test_gradient_h2o16_device_time(lai):
 
 
 def test_gradient_f_shells_vs_finite_differences(lai):
-    """H2O / cc-pVTZ (f on O, d on H): the warp-per-quartet gradient kernel on the
+    """H2O / cc-pVTZ (f on O, d on H): the block-per-quartet gradient kernel on the
     classes above d, and the thread-per-quartet ones on the rest, against central
     differences of our energy (no screening) on three coordinates."""
     w = lai.workloads.make("h2o1_ccpvtz")

@@ -271,8 +271,8 @@ def test_mixed_precision_relative_primitive_cut(lai):
 
 def test_mixed_precision_f_classes_run_fp32(lai):
     """(H2O)2 / cc-pVTZ (f on O) at cut 1e-6: quartets of f classes below the FP32
-    Schwarz cut run in FP32 (the warp-per-quartet FP32 variant; only classes too
-    large for it stay FP64): the FP32 count, checked against the canonical
+    Schwarz cut run in FP32 (the block kernel's FP32 variant; only classes of more
+    than 1024 contracted (e0|f0) integrals stay FP64): the FP32 count, checked against the canonical
     quartets in [threshold, cut) worked out on the host from the engine's Schwarz
     matrix, exceeds what the classes up to d hold, and the energy stays inside the
     1e-8 Eh bar."""

@@ -96,3 +96,35 @@ def test_calls_beside_a_capture_that_is_still_open(call):
                 assert np.max(np.abs(a.cpu().numpy() - b)) < REL * np.max(np.abs(b))
         else:
             assert np.max(np.abs(grad[k].cpu().numpy() - g0)) < 1e-12 * np.max(np.abs(g0))
+
+
+@pytest.mark.parametrize("system", ["alkane6_ccpvtz", "h2o1_ccpvqz"])
+def test_shared_launches_do_not_cost_time(system):
+    """The plain build shares launches among a class's blocks; with a mixed-precision cut
+    below every bound the same quartets run one launch per block."""
+    import time
+
+    import torch
+    if system == "alkane6_ccpvtz":
+        basis = lai.BasisSet.from_atoms(*lai.molecules.alkane(6), "cc-pvtz")
+    else:
+        basis = lai.workloads.make(system).basis
+    eng = lai.Engine(basis)
+    d = torch.from_numpy(lai.molecules.random_density(basis.nbf, 10, np.random.default_rng(0))).cuda()
+    J, K = torch.empty_like(d), torch.empty_like(d)
+    stream = torch.cuda.Stream()
+
+    def ms(cut):
+        best = 1e9
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            eng.jk_device(d.data_ptr(), J.data_ptr(), K.data_ptr(), stream=stream.cuda_stream, fp32_cut=cut)
+            torch.cuda.synchronize()
+            best = min(best, 1e3 * (time.perf_counter() - t))
+        return best
+
+    ms(0.0)
+    shared, single = ms(0.0), ms(1e-25)
+    # launches that fill the device gain nothing by sharing one, and lost 6.6 % by it
+    assert shared < 1.035 * single, (shared, single)
