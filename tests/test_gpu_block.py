@@ -81,3 +81,9 @@ def test_transfer_on_both_sides_keeps_precision(ls):
     # about the first shell's centre on both sides, K' of (3,) is off by 4e-14
     assert np.linalg.norm(J - Jh) < 5e-15 * np.linalg.norm(Jh)
     assert np.linalg.norm(K - Kh) < 1e-14 * np.linalg.norm(Kh)
+
+
+# contracted g, f and d shells on different centres: primitives away from the expansion centre
+@pytest.mark.parametrize("shells", [[(4, 2), (4, 1), (3, 2), (0, 1)], [(4, 1), (3, 3), (2, 3), (2, 2), (1, 2)]])
+def test_contracted_pairs_of_two_centres(shells):
+    test_block_kernel_equals_host_digestion(shells)

@@ -96,3 +96,10 @@ def test_gradient_does_not_depend_on_the_order_of_shells(ls):
         # shell's centre on both sides by 2e-14 to 2e-13
         for g in got[1:]:
             assert np.linalg.norm(g - got[0]) < 1.2e-14 * np.linalg.norm(got[0]), (seed, np.linalg.norm(g - got[0]))
+
+
+# pairs of g and f shells on different centres: 165 rows about the charge, contracted shells
+# whose other primitives lie away from it, kets that stay about their first shell
+@pytest.mark.parametrize("shells", [[(4, 1), (4, 1), (3, 1)], [(4, 1), (3, 2), (4, 1), (2, 2), (2, 1)]])
+def test_gradient_of_two_centre_pairs(shells):
+    test_gradient_matches_differences(shells)
